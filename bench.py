@@ -97,11 +97,10 @@ def add_speedups(res: dict, key: str = "seconds") -> None:
         if "mg_fp64" in res and name in res:
             res[name]["speedup_vs_mg_fp64"] = res["mg_fp64"][key] / res[name][key]
 KERNEL_NAMES = {"tensor": "apply_mma_kernel<Shape<3,4,Elasticity>> (FP64 mma.sync m8n8k4, element-centric)",
-                "face": "vol_mma_kernel + face_mma_kernel<Shape<3,4,Elasticity>> (FP64 mma.sync m8n8k4, "
-                        "face-centric; roofline over both launches of one apply)",
-                "face2": "vol2_kernel + face2_kernel<Shape<3,4,Elasticity>> (FP64 mma.sync m8n8k4, face-centric, "
-                         "cp.async double-buffered coefficient blocks, tile-ordered geometry; roofline over both "
-                         "launches of one apply)",
+                "face": "volw_kernel + facew_kernel<Shape<3,4,Elasticity>> (FP64 mma.sync m8n8k4, face-centric, one warp per "
+                        "8 elements / facets; roofline over both launches of one apply)",
+                "face2": "volw_kernel + facew_kernel<Shape<3,4,Elasticity>> (FP64 mma.sync m8n8k4, face-centric, one warp per "
+                         "8 elements / facets; roofline over both launches of one apply)",
                 "simt": "apply_kernel<Shape<3,4,Elasticity>, double> (SIMT)"}
 
 

@@ -171,26 +171,26 @@ int tdg_bjacobi_blocks(tdg_op* op, double* out);
 /* --- autotuning (no counterpart in tandem) ---------------------------------------------------- */
 
 typedef struct {
-    int family;       /* 0 = element-centric tensor-core kernel, 1 = SIMT kernel, 2 = face-centric
-                         tensor-core kernels (volume kernel + one pass over the facets), 3 = the
-                         face-centric pair software-pipelined (FP64: asynchronous copies of the next
-                         tile's coefficient blocks, tile-ordered geometry; FP32 runs family 2),
+    int family;       /* 0 = element-centric tensor-core kernel, 1 = SIMT kernel, 2 and 3 = face-centric
+                         tensor-core kernels (volume kernel + one pass over the facets): the same
+                         warp-tile kernels in FP64 (one warp per 8 elements / facets, no barriers; 3
+                         with `tile` != 0 runs the volume term in passes), the mma.sync pair in FP32,
                          4 = FP32 only: family 2 with the volume term on the 5th-generation tensor
                          cores (tcgen05.mma kind::tf32, accumulators in tensor memory; shapes with at
                          most 64 volume points, else family 2) */
-    int ctas_per_sm;  /* persistent CTAs per SM requested (0 = default) */
+    int ctas_per_sm;  /* persistent CTAs per SM requested (0 = default); FP64 families 2 and 3: units of
+                         4 warps of the one CTA per SM */
     int tile;         /* family 3, FP64: volume quadrature points per pass of the volume kernel (its
-                         GEMM tiles are D x tile rows of the volume table); 0 = every point in one
-                         pass where the buffers fit two CTAs per SM, else 24; other families 0 */
+                         GEMM tiles are D x tile rows of the volume table); 0 = the warp-tile volume
+                         kernel; other families 0 */
     double ms;        /* measured time of one apply */
 } tdg_tune_entry;
 
 /* Times the apply of this operator (its own mesh, `nrhs` right-hand sides, `precision`) for each
  * candidate launch configuration -- the tensor-core kernels (element-centric, and the
- * face-centric pair; FP64 also its software-pipelined form, FP32 also the pair with the tcgen05
- * volume kernel) at 1 to 4 persistent CTAs per SM (clipped to the occupancy limit of the
- * shape's tile), the software-pipelined FP64 form also at the tile heights that cover the volume
- * points in 1, 2, 3 and 4 passes, and the SIMT kernel -- with CUDA events on
+ * face-centric pair; FP32 also the pair with the tcgen05 volume kernel) at 1 to 4 persistent CTAs
+ * per SM (clipped to the occupancy limit of the shape's tile), the FP64 face-centric form also at
+ * the tile heights that cover the volume points in 2, 3 and 4 passes, and the SIMT kernel -- with CUDA events on
  * `stream`, and keeps the fastest for later tdg_apply / tdg_solve calls of that precision.
  * entries (optional, up to max_entries) receives every measurement; n_entries their count. */
 int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_entry* entries, int max_entries,
@@ -199,7 +199,7 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
  * explicitly: kernel family as in tdg_tune_entry and persistent CTAs per SM. */
 int tdg_set_apply_config(tdg_op* op, int precision, int family, int ctas_per_sm);
 /* Sets the tile height of family 3 (TDG_FP64 only): volume points per pass of its volume kernel, as
- * tdg_tune_entry.tile; a multiple of 8 (3D) or 4 (2D), or 0 for the automatic layout.  A height whose
+ * tdg_tune_entry.tile; a multiple of 8 (3D) or 4 (2D), or 0 for the warp-tile volume kernel.  A height whose
  * buffers do not fit the shape makes tdg_apply return TDG_E_INVALID. */
 int tdg_set_apply_tile(tdg_op* op, int precision, int points_per_pass);
 

@@ -2,11 +2,12 @@
 // block-Jacobi and the device Krylov drivers.
 #include "../../include/tandem_b200.h"
 #include "host/setup.hpp"
+#include "host/warp_tables.hpp"
 #include "kernels/apply_mma.cuh"
 #include "kernels/apply_tc32.cuh"
 #include "kernels/apply_face.cuh"
 #include "kernels/apply_face_tc32.cuh"
-#include "kernels/apply_face2.cuh"
+#include "kernels/apply_warp.cuh"
 #include "kernels/wave.cuh"
 #include "kernels/dispatch.hpp"
 #include "kernels/krylov.cuh"
@@ -268,9 +269,8 @@ struct tdg_op {
     DevOp<float> op32;
     MmaTiles mma;           // FP64 tensor-pipe apply: packed tables and signature tiles
     Tc32Tiles tc32;         // FP32 tensor-core apply (3xTF32): packed tables and signature tiles
-    FaceTiles face;         // face-centric FP64 apply: facet tiles grouped by (l0, l1, mode)
     FaceTiles face32;       // face-centric FP32 apply: the same grouping with the FP32 tile size
-    TileGeo tgeo;           // software-pipelined face-centric FP64 apply: tile-ordered geometry
+    WarpGeo warp;           // warp-tile FP64 apply: fragment tables, lane-ordered geometry
     // explicit wave operator: basis at the volume points, reference inverse mass, -rhoInv W / |J|
     DevArena arena_wave;
     WaveData wave;
@@ -451,11 +451,6 @@ void facet_tiles(HostOperator const& h, int TE, std::vector<int4>& finfo, std::v
     }
 }
 
-// The face2 facet kernel's geometry rows (see face2_point_swizzle): quads of points with the middle
-// two swapped, rows per field rounded up to the quad, for 8-facet tiles.
-inline bool face2_swizzle_host(int D, int N, int Q) { return mma_tile_elements(D, N, Q) == 8; }
-inline int face2_geo_rows_host(int D, int N, int Q, int nq) { return face2_swizzle_host(D, N, Q) ? (nq + 3) / 4 * 4 : nq; }
-
 // The facet tiles' geometry [tile][field][nq][TE] (n, n_unit, then Poisson K G0, K G1 or
 // elasticity G0, G1, lam0, mu0, lam1, mu1; unused slots zero), the penalty [tile][TE] and the facet
 // and element ids of every slot {facet, side-0 element, side-1 element (-1 unless mode 1), 0}.
@@ -506,54 +501,49 @@ void tile_facet_geometry(HostOperator const& h, int TE, std::vector<int> const& 
     }
 }
 
-// Geometry and coefficients of the software-pipelined face-centric apply (apply_face2.cuh) in tile
-// order: per element tile of TE consecutive elements [field][Nq rows][TE] (J^-1, then the volume
-// coefficients), per facet tile [field][nq rows][TE] (n, n_unit, then Poisson K G0, K G1 or
-// elasticity G0, G1, lam0, mu0, lam1, mu1) and the penalty [TE]; unused slots and padding rows
-// zero; 8-wide tiles hold point q in row face2_point(q) of nq rounded up to 4 rows.  The same values
-// as the reference-layout arrays, read with the tile's elements or facets fastest.
-int upload_tile_geometry(tdg_op* op, DevArena& arena, std::vector<int> const& fids, std::vector<int4> const& ftiles) {
+// Tables and geometry of the warp-tile apply: facet tiles of 8 facets of one key, volume tiles of 8
+// consecutive elements.
+int upload_warp(tdg_op* op, DevArena& arena) {
     auto const& h = op->h;
-    const int D = h.D, DD = D * D, Nq = h.Nq;
-    const int TE = mma_tile_elements(D, h.N, h.Q);
-    const bool poisson = h.kind == 0;
-    const int ncoef = poisson ? 1 : 2;
-    const int vf = DD + ncoef;
-    const int64_t vtiles = (h.E + TE - 1) / TE;
-    // rows per field and the row of point q (the volume kernel's point swizzle)
-    const bool swz = face2_swizzle_host(D, h.N, h.Q);
-    const int Nqg = face2_geo_rows_host(D, h.N, h.Q, Nq);
-    std::vector<double> vol(static_cast<size_t>(vtiles) * vf * Nqg * TE, 0.0);
+    WarpGeo wg;
+    std::vector<int4> finfo, ftiles;
+    std::vector<int> fids;
+    facet_tiles(h, 8, finfo, fids, ftiles);
+    const WarpFacetTables ft = warp_facet_tables(h);
+    const int64_t nft = static_cast<int64_t>(ftiles.size()), fs = warp_facet_stride(h);
+    std::vector<double> fct(static_cast<size_t>(nft) * fs, 0.0);
+    std::vector<int4> tids(static_cast<size_t>(nft) * 8, make_int4(-1, -1, -1, 0));
 #pragma omp parallel for schedule(static)
-    for (int64_t e = 0; e < h.E; ++e) {
-        const int64_t t = e / TE;
-        const int te = static_cast<int>(e % TE);
-        double* base = &vol[static_cast<size_t>(t) * vf * Nqg * TE];
-        for (int c = 0; c < DD; ++c)
-            for (int q = 0; q < Nq; ++q)
-                base[(static_cast<size_t>(c) * Nqg + (swz ? face2_point(q) : q)) * TE + te] =
-                    h.vG[(static_cast<size_t>(e) * DD + c) * Nq + q];
-        for (int c = 0; c < ncoef; ++c)
-            for (int q = 0; q < Nq; ++q)
-                base[(static_cast<size_t>(DD + c) * Nqg + (swz ? face2_point(q) : q)) * TE + te] =
-                    h.vCoef[(static_cast<size_t>(e) * ncoef + c) * Nq + q];
+    for (int64_t t = 0; t < nft; ++t) {
+        const int4 td = ftiles[t];
+        warp_facet_tile(h, &fids[td.x], td.y, &fct[static_cast<size_t>(t) * fs]);
+        for (int te = 0; te < td.y; ++te) {
+            const int f = fids[td.x + te];
+            tids[static_cast<size_t>(t) * 8 + te] =
+                make_int4(f, static_cast<int>(h.up[2 * f]), (td.z >> 4) == 1 ? static_cast<int>(h.up[2 * f + 1]) : -1, 0);
+        }
     }
-    const size_t nft = ftiles.size();
-    std::vector<double> fct, pen;
-    std::vector<int4> tids;
-    tile_facet_geometry(h, TE, fids, ftiles, fct, pen, tids, face2_geo_rows_host(h.D, h.N, h.Q, h.nq),
-                        face2_swizzle_host(h.D, h.N, h.Q));
-    if (nft) TDG_CUDA_TRY(arena.upload(&op->face.tids, tids));
+    const int64_t nvt = (h.E + 7) / 8, vs = warp_volume_stride(h);
+    std::vector<double> vol(static_cast<size_t>(nvt) * vs, 0.0);
+#pragma omp parallel for schedule(static)
+    for (int64_t t = 0; t < nvt; ++t) warp_volume_tile(h, t, &vol[static_cast<size_t>(t) * vs]);
+    if (nft) {
+        TDG_CUDA_TRY(arena.upload(&wg.fct, fct));
+        TDG_CUDA_TRY(arena.upload(&wg.ftiles, ftiles));
+        TDG_CUDA_TRY(arena.upload(&wg.tids, tids));
+    }
+    wg.face_tables = ft.tables;
+    TDG_CUDA_TRY(arena.upload(&wg.ftab, ft.frags));
+    TDG_CUDA_TRY(arena.upload(&wg.fperm, ft.perm));
+    TDG_CUDA_TRY(arena.upload(&wg.vtab, warp_volume_frags(h)));
+    TDG_CUDA_TRY(arena.upload(&wg.vol, vol));
     {
         const int* st = nullptr;
         TDG_CUDA_TRY(arena.upload(&st, std::vector<int>(1, 0)));
-        op->tgeo.status = const_cast<int*>(st);
+        wg.status = const_cast<int*>(st);
     }
-    TDG_CUDA_TRY(arena.upload(&op->tgeo.vol, vol));
-    if (nft) {
-        TDG_CUDA_TRY(arena.upload(&op->tgeo.fct, fct));
-        TDG_CUDA_TRY(arena.upload(&op->tgeo.pen, pen));
-    }
+    wg.nftiles = static_cast<int>(nft);
+    op->warp = wg;
     return 0;
 }
 
@@ -585,17 +575,11 @@ int upload_mma(tdg_op* op, DevArena& arena) {
     op->mma.ntiles = static_cast<int>(tiles.size());
     op->mma.table_doubles = static_cast<int>(tab.size());
 
-    std::vector<int4> finfo, ftiles;
-    std::vector<int> fids;
-    facet_tiles(h, mma_tile_elements(D, h.N, h.Q), finfo, fids, ftiles);
-    if (!fids.empty()) {
-        TDG_CUDA_TRY(arena.upload(&op->face.fperm, fids));
-        TDG_CUDA_TRY(arena.upload(&op->face.ftiles, ftiles));
+    try {
+        TDG_TRY(upload_warp(op, arena));
+    } catch (std::exception const& e) {
+        return fail(TDG_E_NOMEM, std::string("warp-tile tables: ") + e.what());
     }
-    TDG_CUDA_TRY(arena.upload(&op->face.finfo, finfo));
-    op->face.nftiles = static_cast<int>(ftiles.size());
-    op->face.tables = op->mma.tables + static_cast<size_t>(MV) * LDT;
-    TDG_TRY(upload_tile_geometry(op, arena, fids, ftiles));
     return 0;
 }
 
@@ -1526,18 +1510,19 @@ int tdg_apply(tdg_op* op, int precision, const void* x, void* y, int nrhs, int64
     int rc = TDG_E_INVALID;
     const int pi = precision == TDG_FP64 ? 0 : 1;
     const bool tensor = op->use_mma && op->family[pi] == 0;
-    if (precision == TDG_FP64 && op->use_mma && op->family[0] == 3)
-        rc = launch_apply_face2(h.D, h.N, h.kind, op->op64, op->mma, op->face, op->tgeo,
-                                static_cast<const double*>(x), static_cast<double*>(y), nrhs, ld, s, op->ctas[0],
-                                op->tile[0]);
-    // family 3 falls back to family 2 only where its automatic layout does not fit; an explicit
-    // points-per-pass that does not fit is the caller's error
-    if (precision == TDG_FP64 && op->family[0] == 3 && op->tile[0] != 0 && rc == TDG_E_INVALID)
-        return fail(rc, "points per pass do not fit this shape");
-    if (precision == TDG_FP64 && op->use_mma && (op->family[0] == 2 || (op->family[0] == 3 && rc == TDG_E_INVALID)))
-        rc = launch_apply_face(h.D, h.N, h.kind, op->op64, op->mma, op->face, static_cast<const double*>(x),
-                               static_cast<double*>(y), nrhs, ld, s, op->ctas[0]);
-    else if (precision == TDG_FP64 && tensor)
+    if (precision == TDG_FP64 && op->use_mma && op->family[0] >= 2) {
+        // the warp-tile kernels; family 3 with points per pass runs the volume kernel in passes
+        const double* xd = static_cast<const double*>(x);
+        double* yd = static_cast<double*>(y);
+        if (op->family[0] == 3 && op->tile[0] != 0) {
+            rc = launch_vol2(h.D, h.N, h.kind, h.E, h.Nq, op->mma.tables, op->warp, xd, yd, nrhs, ld, s, op->ctas[0],
+                             op->tile[0]);
+            if (rc == TDG_E_INVALID) return fail(rc, "points per pass do not fit this shape");
+        } else {
+            rc = launch_volume_warp(h.D, h.N, h.kind, h.E, h.Nq, op->warp, xd, yd, nrhs, ld, s, op->ctas[0]);
+        }
+        if (rc == 0) rc = launch_facets_warp(h.D, h.N, h.kind, h.nq, op->warp, xd, yd, nrhs, ld, s, op->ctas[0]);
+    } else if (precision == TDG_FP64 && tensor)
         rc = launch_apply_mma(h.D, h.N, h.kind, op->op64, op->mma, static_cast<const double*>(x),
                               static_cast<double*>(y), nrhs, ld, s, op->ctas[0]);
     if (precision == TDG_FP64 && rc == TDG_E_INVALID)
@@ -1710,11 +1695,12 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
     std::vector<Cand> cands;
     if (op->use_mma)
         for (int c = 1; c <= 4; ++c) cands.push_back({0, c, 0});
-    if (op->use_mma)
+    if (op->use_mma && precision == TDG_FP32)
         for (int c = 1; c <= 4; ++c) cands.push_back({2, c, 0});
-    if (op->use_mma && precision == TDG_FP64)
-        for (int c = 1; c <= 2; ++c)
-            for (int t : face2_tile_candidates(h.D, h.Nq)) cands.push_back({3, c, t});
+    if (op->use_mma && precision == TDG_FP64)  // families 2 and 3 are the same kernels in FP64
+        for (int c = 1; c <= 4; ++c)
+            for (int t : face2_tile_candidates(h.D, h.Nq))
+                if (t == 0 || c <= 2) cands.push_back({3, c, t});
     if (op->use_mma && precision == TDG_FP32)  // the facet kernel's CTAs; the tcgen05 volume kernel runs one per SM
         for (int c = 1; c <= 4; ++c) cands.push_back({4, c, 0});
     cands.push_back({1, 0, 0});
@@ -2482,7 +2468,7 @@ int solve_segments(tdg_op* op, const double* b, double* x, std::vector<int64_t> 
     stats->converged = (!diverged && worst <= rtol) ? 1 : 0;
     if (op->pc == TDG_PC_MG) TDG_TRY(mg_check_coarse(op, s));
     if (diverged) return fail(TDG_E_DIVERGED, "non-finite residual in the Krylov iteration");
-    for (int* word : {op->tgeo.status, op->tc32.status})
+    for (int* word : {op->warp.status, op->tc32.status})
         if (word) {  // a bounded wait of a pipelined kernel that ran out makes the solve invalid
             int st = 0;
             TDG_CUDA_TRY(cudaMemcpy(&st, word, sizeof st, cudaMemcpyDeviceToHost));

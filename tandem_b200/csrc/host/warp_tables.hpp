@@ -1,0 +1,31 @@
+// Host-side data of the warp-tile FP64 apply (kernels/apply_warp.cuh): B fragments of the basis
+// tables in mma order and per-point geometry in lane order.
+#pragma once
+
+#include "setup.hpp"
+
+#include <cstdint>
+#include <vector>
+
+namespace tdg {
+
+struct WarpFacetTables {
+    std::vector<double> frags;  // [table][fragment][lane]
+    int tables = 0;             // 1: all faces share one table (nodal bases); else one per face
+    std::vector<int> perm;      // [face][8 NT]
+};
+// Facet fragments per local face and the order of the basis functions on it (face functions first).
+WarpFacetTables warp_facet_tables(HostOperator const& h);
+
+// Volume fragments.
+std::vector<double> warp_volume_frags(HostOperator const& h);
+// Volume geometry of the tile of elements [8 tile, 8 tile + 8): warp_volume_stride(h) doubles, zeroed.
+int64_t warp_volume_stride(HostOperator const& h);
+void warp_volume_tile(HostOperator const& h, int64_t tile, double* out);
+
+// Facet geometry of one tile of up to 8 facets of one (l0, l1): `count` facet ids at `fids`; out
+// holds warp_facet_stride(h) doubles, zeroed.
+int64_t warp_facet_stride(HostOperator const& h);
+void warp_facet_tile(HostOperator const& h, int const* fids, int count, double* out);
+
+}  // namespace tdg

@@ -7,7 +7,6 @@
 
 #include "apply_face.cuh"
 #include "apply_tc32.cuh"
-#include "apply_face2.cuh"  // face2_point
 
 namespace tdg {
 

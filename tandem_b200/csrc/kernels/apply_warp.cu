@@ -1,0 +1,166 @@
+// Instances and launchers of the warp-tile FP64 apply (apply_warp.cuh).
+#include "apply_warp.cuh"
+#include "dispatch.hpp"
+
+#include "../../../include/tandem_b200.h"
+
+#include <algorithm>
+
+namespace tdg {
+
+namespace {
+
+// Dynamic shared memory a CTA may take beside the kernels' static arrays.
+size_t shared_limit() {
+    int dev = 0, optin = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    return optin > 2048 ? static_cast<size_t>(optin) - 2048 : 0;
+}
+
+// Grid, warps per CTA (one persistent CTA per SM) and split of `nwork` items of `nblk` blocks each.
+struct Plan {
+    int grid, warps;
+    WarpSplit split;
+};
+// most: warps the launch bound and shared memory allow; ctas: the caller's limit (4 warps each, 0
+// none); mma: products of an item.  A last round that fills less than 85 % of the warps is split (a
+// whole-item round of 8 warps then costs about as much as its split form: 41 k clocks at 3D p4
+// elasticity).  Items of fewer than 256 products (4 k clocks of the FP64 pipe) stay whole: their
+// time is the latency of their loads, which every part would pay again.
+Plan make_plan(int most, int64_t nwork, int nblk, int mma, int ctas) {
+    const int sms = device_sm_count();
+    Plan p;
+    if (ctas > 0) most = std::min(most, 4 * ctas);
+    if (mma < 256) nblk = 1;
+    const int64_t share = (nwork + sms - 1) / sms;  // items per SM
+    p.warps = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, share * nblk)));
+    p.grid = static_cast<int>(std::min<int64_t>(sms, nwork));
+    const int64_t all = static_cast<int64_t>(p.grid) * p.warps, rest = nwork % all;
+    p.split.whole = nwork - rest;
+    p.split.parts = std::min(nblk, p.warps);
+    if (rest * 100 >= all * 85 || p.split.parts == 1) p.split.whole = nwork + (rest ? all - rest : 0);
+    return p;
+}
+
+template <class K>
+int allow_shared(K kern, bool& ready) {
+    if (ready) return 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared_limit())) !=
+        cudaSuccess)
+        return TDG_E_CUDA;
+    ready = true;
+    return 0;
+}
+
+template <class S, bool TG>
+int launch_facets(int nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld, cudaStream_t s,
+                  int ctas, int most, size_t tab, size_t per_warp) {
+    static bool ready = false;
+    auto kern = facew_kernel<S, TG>;
+    if (int rc = allow_shared(kern, ready)) return rc;
+    const int64_t nwork = static_cast<int64_t>(wg.nftiles) * nrhs;
+    Plan p = make_plan(most, nwork, WarpBlocks(nq).count(), 2 * S::Q * warp_facet_frags<S>(nq), ctas);
+    p.split.whole = std::min(p.split.whole, nwork);
+    kern<<<p.grid, 32 * p.warps, tab + p.warps * per_warp, s>>>(nq, wg, p.split, x, y, ld, nrhs);
+    return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;
+}
+
+template <class S>
+int run_facets(int nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld, cudaStream_t s, int ctas) {
+    using L = WarpTile<S>;
+    if (wg.nftiles == 0) return 0;
+    const size_t limit = shared_limit();
+    const size_t tab = sizeof(double) * 32 * static_cast<size_t>(wg.face_tables) * warp_facet_frags<S>(nq);
+    const size_t per_warp = sizeof(double) * facet_warp_doubles<S>(nq);
+    if (per_warp > limit) return TDG_E_INVALID;
+    const bool fits = tab + 4 * per_warp <= limit;
+    const int most = static_cast<int>(std::min<size_t>(L::FWARPS, (limit - (fits ? tab : 0)) / per_warp));
+    if (fits) return launch_facets<S, false>(nq, wg, x, y, nrhs, ld, s, ctas, most, tab, per_warp);
+    return launch_facets<S, true>(nq, wg, x, y, nrhs, ld, s, ctas, most, 0, per_warp);
+}
+
+template <class S, bool TG>
+int launch_volume(int64_t E, int Nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld,
+                  cudaStream_t s, int ctas, int most, size_t tab, size_t per_warp) {
+    static bool ready = false;
+    auto kern = volw_kernel<S, TG>;
+    if (int rc = allow_shared(kern, ready)) return rc;
+    const int64_t nwork = (E + 7) / 8 * nrhs;
+    const Plan p = make_plan(most, nwork, WarpBlocks(Nq).count(), S::Q * warp_volume_frags<S>(Nq), ctas);
+    const size_t smem = tab + (p.split.whole < nwork ? p.warps * per_warp : 0);
+    kern<<<p.grid, 32 * p.warps, smem, s>>>(E, Nq, wg, p.split, x, y, ld, nrhs);
+    return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;
+}
+
+template <class S>
+int run_volume(int64_t E, int Nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld, cudaStream_t s,
+               int ctas) {
+    using L = WarpTile<S>;
+    const size_t limit = shared_limit();
+    const size_t tab = sizeof(double) * 32 * static_cast<size_t>(warp_volume_frags<S>(Nq));
+    const size_t per_warp = sizeof(double) * volume_warp_doubles<S>();
+    if (tab + 4 * per_warp <= limit) {
+        const int most = static_cast<int>(std::min<size_t>(L::VWARPS, (limit - tab) / per_warp));
+        return launch_volume<S, false>(E, Nq, wg, x, y, nrhs, ld, s, ctas, most, tab, per_warp);
+    }
+    return launch_volume<S, true>(E, Nq, wg, x, y, nrhs, ld, s, ctas, L::VWARPS, 0, per_warp);
+}
+
+template <int D, int N>
+int volume_kind(int kind, int64_t E, int Nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld,
+                cudaStream_t s, int ctas) {
+    if (kind == kPoisson) return run_volume<Shape<D, N, kPoisson>>(E, Nq, wg, x, y, nrhs, ld, s, ctas);
+    return run_volume<Shape<D, N, kElasticity>>(E, Nq, wg, x, y, nrhs, ld, s, ctas);
+}
+
+template <int D>
+int volume_deg(int N, int kind, int64_t E, int Nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld,
+               cudaStream_t s, int ctas) {
+    switch (N) {
+        case 1: return volume_kind<D, 1>(kind, E, Nq, wg, x, y, nrhs, ld, s, ctas);
+        case 2: return volume_kind<D, 2>(kind, E, Nq, wg, x, y, nrhs, ld, s, ctas);
+        case 3: return volume_kind<D, 3>(kind, E, Nq, wg, x, y, nrhs, ld, s, ctas);
+        case 4: return volume_kind<D, 4>(kind, E, Nq, wg, x, y, nrhs, ld, s, ctas);
+        default: return TDG_E_INVALID;
+    }
+}
+
+template <int D, int N>
+int facets_kind(int kind, int nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld, cudaStream_t s,
+                int ctas) {
+    if (kind == kPoisson) return run_facets<Shape<D, N, kPoisson>>(nq, wg, x, y, nrhs, ld, s, ctas);
+    return run_facets<Shape<D, N, kElasticity>>(nq, wg, x, y, nrhs, ld, s, ctas);
+}
+
+template <int D>
+int facets_deg(int N, int kind, int nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld,
+               cudaStream_t s, int ctas) {
+    switch (N) {
+        case 1: return facets_kind<D, 1>(kind, nq, wg, x, y, nrhs, ld, s, ctas);
+        case 2: return facets_kind<D, 2>(kind, nq, wg, x, y, nrhs, ld, s, ctas);
+        case 3: return facets_kind<D, 3>(kind, nq, wg, x, y, nrhs, ld, s, ctas);
+        case 4: return facets_kind<D, 4>(kind, nq, wg, x, y, nrhs, ld, s, ctas);
+        default: return TDG_E_INVALID;
+    }
+}
+
+}  // namespace
+
+int launch_facets_warp(int D, int N, int kind, int nq, WarpGeo const& wg, const double* x, double* y, int nrhs,
+                       int64_t ld, cudaStream_t s, int ctas) {
+    if (nrhs < 1 || (wg.nftiles > 0 && (!wg.ftab || !wg.fct))) return TDG_E_INVALID;
+    if (D == 2) return facets_deg<2>(N, kind, nq, wg, x, y, nrhs, ld, s, ctas);
+    if (D == 3) return facets_deg<3>(N, kind, nq, wg, x, y, nrhs, ld, s, ctas);
+    return TDG_E_INVALID;
+}
+
+int launch_volume_warp(int D, int N, int kind, int64_t E, int Nq, WarpGeo const& wg, const double* x, double* y,
+                       int nrhs, int64_t ld, cudaStream_t s, int ctas) {
+    if (nrhs < 1 || !wg.vtab || !wg.vol) return TDG_E_INVALID;
+    if (D == 2) return volume_deg<2>(N, kind, E, Nq, wg, x, y, nrhs, ld, s, ctas);
+    if (D == 3) return volume_deg<3>(N, kind, E, Nq, wg, x, y, nrhs, ld, s, ctas);
+    return TDG_E_INVALID;
+}
+
+}  // namespace tdg

@@ -24,22 +24,20 @@ struct MmaTiles;
 int launch_apply_mma(int D, int N, int kind, DevOp<double> const& op, MmaTiles const& mt, const double* x, double* y,
                      int nrhs, int64_t ld, cudaStream_t s, int ctas = 0);
 
-// Face-centric FP64 apply (apply_face.cuh): volume kernel (y = volume term) then facet kernel
-// (y += facet terms, each facet once for both sides).
+// Warp-tile FP64 apply (apply_warp.cuh): volume term (stores y) and facet terms (added into y).
+// ctas: 4 warps per SM for each (0 = as many as the shape's registers and shared memory allow).
+struct WarpGeo;
+int launch_volume_warp(int D, int N, int kind, int64_t E, int Nq, WarpGeo const& wg, const double* x, double* y,
+                       int nrhs, int64_t ld, cudaStream_t s, int ctas = 0);
+int launch_facets_warp(int D, int N, int kind, int nq, WarpGeo const& wg, const double* x, double* y, int nrhs,
+                       int64_t ld, cudaStream_t s, int ctas = 0);
 struct FaceTiles;
-int launch_apply_face(int D, int N, int kind, DevOp<double> const& op, MmaTiles const& mt, FaceTiles const& ft,
-                      const double* x, double* y, int nrhs, int64_t ld, cudaStream_t s, int ctas = 0);
 
-// Software-pipelined face-centric FP64 apply (apply_face2.cuh): cp.async double-buffered
-// coefficient blocks, tile-ordered geometry (TileGeo), both sides' fluxes from one stress.
-struct TileGeo;
-// qc: volume points per pass of the volume kernel (the M extent of its GEMM tiles is D x qc rows);
-// 0 = every point in one pass where the buffers fit two CTAs per SM, else 24; otherwise a multiple
-// of face2_pass_step(D) (TDG_E_INVALID else).
-int launch_apply_face2(int D, int N, int kind, DevOp<double> const& op, MmaTiles const& mt, FaceTiles const& ft,
-                       TileGeo const& tg, const double* x, double* y, int nrhs, int64_t ld, cudaStream_t s,
-                       int ctas = 0, int qc = 0);
-// Granularity of qc: passes start on whole 8-row GEMM tiles and on whole point quads.
+// The volume term in passes of qc points (apply_face2.cuh), a multiple of face2_pass_step(D);
+// TDG_E_INVALID where its buffers do not fit.
+int launch_vol2(int D, int N, int kind, int64_t E, int Nq, const double* tables, WarpGeo const& wg, const double* x,
+                double* y, int nrhs, int64_t ld, cudaStream_t s, int ctas, int qc);
+// Granularity of qc: passes start on whole 8-row GEMM tiles.
 constexpr int face2_pass_step(int D) { return D == 3 ? 8 : 4; }
 
 // Face-centric FP32 apply (apply_face_tc32.cuh), TX = float or double vectors.
