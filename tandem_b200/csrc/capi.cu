@@ -4,6 +4,7 @@
 #include "host/setup.hpp"
 #include "host/warp_tables.hpp"
 #include "kernels/apply_mma.cuh"
+#include "kernels/bjacobi.cuh"
 #include "kernels/apply_tc32.cuh"
 #include "kernels/apply_face.cuh"
 #include "kernels/apply_face_tc32.cuh"
@@ -1223,7 +1224,7 @@ int mg_setup_aux(tdg_op* op, cudaStream_t s) {
     }
     const double* ddiag = nullptr;
     TDG_CUDA_TRY(mg.arena.upload(&ddiag, diag));
-    TDG_CUDA_TRY(mg.arena.alloc(&mg.cinv, diag.size()));
+    TDG_CUDA_TRY(mg.arena.alloc(&mg.cinv, static_cast<size_t>(nv) * bjac_packed_size(Q)));
     return mgk(launch_bjac_invert<double>(Q, nv, ddiag, mg.cinv, mg.status, s), "P1 block inversion");
 }
 
@@ -1320,7 +1321,7 @@ int mg_setup(tdg_op* op, tdg_mg_opts o, cudaStream_t s) {
         TDG_CUDA_TRY(cudaMalloc(&blk0, sizeof(double) * E * L0.bs * L0.bs));
         int rc = mgk(launch_mg_self_blocks(E, mg.NB, L0.bs, L0.A, blk0, s), "coarse blocks");
         if (!rc) {
-            cudaError_t ce = mg.arena.alloc(&mg.cinv, static_cast<size_t>(E) * L0.bs * L0.bs);
+            cudaError_t ce = mg.arena.alloc(&mg.cinv, static_cast<size_t>(E) * bjac_packed_size(L0.bs));
             rc = ce == cudaSuccess ? 0 : fail(TDG_E_NOMEM, "multigrid: coarse inverses");
         }
         if (!rc) rc = mgk(launch_bjac_invert<double>(L0.bs, E, blk0, mg.cinv, mg.status, s), "coarse inversion");
@@ -1764,7 +1765,7 @@ int tdg_bjacobi_setup(tdg_op* op, int precision, void* stream) {
     if (precision != TDG_FP64 && precision != TDG_FP32) return fail(TDG_E_INVALID, "bad precision");
     auto const& h = op->h;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const size_t nblk = static_cast<size_t>(h.E) * h.bs * h.bs;
+    const size_t nblk = static_cast<size_t>(h.E) * bjac_packed_size(h.bs);
     TDG_TRY(ensure_blocks(op, s));
     if (op->inv && op->inv_precision == precision) return 0;
     if (op->inv) {

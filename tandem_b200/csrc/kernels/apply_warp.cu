@@ -12,10 +12,13 @@ namespace {
 
 // Dynamic shared memory a CTA may take beside the kernels' static arrays.
 size_t shared_limit() {
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    return optin > 2048 ? static_cast<size_t>(optin) - 2048 : 0;
+    static const size_t limit = [] {
+        int dev = 0, optin = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        return optin > 2048 ? static_cast<size_t>(optin) - 2048 : size_t(0);
+    }();
+    return limit;
 }
 
 // Grid, warps per CTA (one persistent CTA per SM) and split of `nwork` items of `nblk` blocks each.

@@ -4,6 +4,8 @@
 
 #include "../../../include/tandem_b200.h"
 
+#include <type_traits>
+
 namespace tdg {
 
 namespace {
@@ -49,16 +51,60 @@ int run_invert(int64_t E, const double* blk, T* inv, int* status, cudaStream_t s
     return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;
 }
 
-template <int BS, typename TM, typename TV>
-int run_bapply(int64_t E, const TM* inv, const TV* r, TV* z, int nrhs, int64_t ld, cudaStream_t s) {
+template <int BS, typename TM, typename TV, int RB>
+int run_rows(int64_t E, const TM* inv, const TV* r, TV* z, int nrhs, int64_t ld, cudaStream_t s) {
     constexpr int TE = (256 / BS) > 0 ? (256 / BS) : 1;
     const int64_t ntiles = (E + TE - 1) / TE;
     int64_t grid = static_cast<int64_t>(device_sm_count()) * 8;
     if (grid > ntiles) grid = ntiles;
     if (grid < 1) grid = 1;
-    dim3 g(static_cast<unsigned>(grid), static_cast<unsigned>(nrhs));
-    bjac_apply_kernel<BS, TM, TV><<<g, 256, 0, s>>>(E, inv, r, z, ld);
+    dim3 g(static_cast<unsigned>(grid), static_cast<unsigned>((nrhs + RB - 1) / RB));
+    bjac_apply_kernel<BS, TM, TV, RB><<<g, 256, 0, s>>>(E, inv, r, z, nrhs, ld);
     return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;
+}
+
+template <int BS, typename TM, typename TV>
+int run_stream(int64_t E, const TM* inv, const TV* r, TV* z, cudaStream_t s) {
+    using L = BjacStream<BS, TM>;
+    constexpr size_t smem = L::smem(sizeof(TV));
+    auto kern = bjac_stream_kernel<BS, TM, TV>;
+    static int per_sm = 0;
+    if (per_sm == 0) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
+            cudaSuccess)
+            return TDG_E_CUDA;
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 256, smem) != cudaSuccess || n < 1) n = 1;
+        per_sm = n;
+    }
+    const int64_t pairs = ((E + L::TE - 1) / L::TE + 1) / 2;  // two teams per CTA
+    int64_t grid = static_cast<int64_t>(device_sm_count()) * per_sm;
+    if (grid > pairs) grid = pairs;
+    kern<<<static_cast<unsigned>(grid), 256, smem, s>>>(E, inv, r, z);
+    return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;
+}
+
+// Inverses up to this size stay in L2 and a row's second access costs nothing: 8,192 blocks of 15
+// (7.9 MB) 3.98 us by rows, 4.27 us streamed; 10,368 blocks of 105 (462 MB) 172 and 120 us.
+constexpr int64_t kStreamBytes = int64_t(32) << 20;
+
+// One right-hand side: bound by the inverses, streamed.  Several: FP64 vectors on the tensor pipe from
+// blocks of 10 (below, a fragment is mostly padding); else four columns per row.
+template <int BS, typename TM, typename TV>
+int run_bapply(int64_t E, const TM* inv, const TV* r, TV* z, int nrhs, int64_t ld, cudaStream_t s) {
+    if (nrhs == 1 && E * bjac_packed_size(BS) * static_cast<int64_t>(sizeof(TM)) >= kStreamBytes)
+        return run_stream<BS, TM, TV>(E, inv, r, z, s);
+    if (nrhs == 1) return run_rows<BS, TM, TV, 1>(E, inv, r, z, nrhs, ld, s);
+    if constexpr (std::is_same_v<TV, double> && BS >= 10) {
+        constexpr int cols = 8 * bjac_mma_tiles<BS>();
+        int64_t grid = static_cast<int64_t>(device_sm_count()) * 16;
+        if (grid > (E + 3) / 4) grid = (E + 3) / 4;
+        dim3 g(static_cast<unsigned>(grid), static_cast<unsigned>((nrhs + cols - 1) / cols));
+        bjac_mma_kernel<BS, TM><<<g, 128, 0, s>>>(E, inv, r, z, nrhs, ld);
+        return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;
+    } else {
+        return run_rows<BS, TM, TV, 4>(E, inv, r, z, nrhs, ld, s);
+    }
 }
 
 // Block sizes bs = binom(N + D, D) * Q for D in {2, 3}, N in [1, 4], Q in {1, D}.

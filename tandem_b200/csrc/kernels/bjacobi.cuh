@@ -8,12 +8,23 @@
 //   column-major: blk[e][col * BS + row], row = k + NBF p.
 // invert: Gauss-Jordan without pivoting in shared memory; a non-positive pivot marks the block
 //   as not positive definite (SIPG diagonal blocks are SPD for a sufficient penalty).
-// apply: z_e = D_e^-1 r_e, one thread per (element, row), inverse streamed column by column.
+// apply: z_e = D_e^-1 r_e.  The apply is bound by reading the inverses, so they are stored as the
+//   half that symmetry leaves: entry (i, (i + d) mod BS) for every row i and d = 0 .. BS / 2, d-major
+//   (odd sizes hold every pair once, even ones the pairs of d = BS / 2 twice).  A row then takes two
+//   entries per d, both contiguous over the rows: its own and that of row i - d; the block is staged
+//   in shared memory, because the second access through L1 cost what the halved bytes gave.
+//   Several FP64 right-hand sides go through the FP64 tensor pipe, one warp per element, the inverse
+//   read once per 8 to 32 columns.
 #pragma once
 
+#include "apply_mma.cuh"
+#include "async.cuh"
 #include "common.cuh"
 
 namespace tdg {
+
+// Entries of a packed symmetric BS x BS inverse, padded to whole 16 bytes in FP32 and FP64.
+__host__ __device__ constexpr int bjac_packed_size(int bs) { return ((bs / 2 + 1) * bs + 3) / 4 * 4; }
 
 template <class S>
 __host__ __device__ inline int bjac_assemble_smem_doubles(int Nq, int nq) {
@@ -147,7 +158,7 @@ __global__ void __launch_bounds__(256) bjac_assemble_kernel(DevOp<double> op, do
     }
 }
 
-// In-place Gauss-Jordan inversion of one BS x BS block per CTA; writes the inverse in T.
+// In-place Gauss-Jordan inversion of one BS x BS block per CTA; writes the packed inverse in T.
 template <int BS, typename T>
 __global__ void __launch_bounds__(256)
     bjac_invert_kernel(const double* __restrict__ blk, T* __restrict__ inv, int* __restrict__ status) {
@@ -181,36 +192,186 @@ __global__ void __launch_bounds__(256)
         }
         __syncthreads();
     }
-    for (int i = tid; i < BS * BS; i += blockDim.x) inv[e * BS * BS + i] = static_cast<T>(a[i]);
+    constexpr int PK = bjac_packed_size(BS);
+    for (int i = tid; i < PK; i += blockDim.x) {
+        const int d = i / BS, row = i % BS;
+        inv[e * PK + i] = d <= BS / 2 ? static_cast<T>(a[(row + d) % BS * BS + row]) : T(0);
+    }
     if (tid == 0 && bad) atomicOr(status, 1);
 }
 
-// z = Dinv r for nrhs vectors: one thread per (element, row).
+// Entries d0 <= d < d1 of one row of Dinv r, added to s: m the packed inverse's row d0 at this row, rv
+// the vector at this row, held twice in a row (no wrap of row + d) with RB copies 2 BS apart.
+template <int BS, typename TM, typename TV, int RB>
+__device__ __forceinline__ void bjac_row(const TM* m, const TV* rv, int row, int d0, int d1, TV (&s)[RB]) {
+    m -= d0 * BS;
+    if (d0 == 0) {
+#pragma unroll
+        for (int j = 0; j < RB; ++j) s[j] += static_cast<TV>(m[0]) * rv[j * 2 * BS];
+        d0 = 1;
+    }
+    const int pairs = d1 < (BS + 1) / 2 ? d1 : (BS + 1) / 2;
+#pragma unroll 8
+    for (int d = d0; d < pairs; ++d) {
+        const TV a = static_cast<TV>(m[d * BS]);
+        const TV b = static_cast<TV>(m[d * BS - d + (row < d ? BS : 0)]);
+#pragma unroll
+        for (int j = 0; j < RB; ++j) s[j] += a * rv[j * 2 * BS + d] + b * rv[j * 2 * BS + BS - d];
+    }
+    if (BS % 2 == 0 && d1 > BS / 2) {  // held for both rows of the pair
+        const TV a = static_cast<TV>(m[BS / 2 * BS]);
+#pragma unroll
+        for (int j = 0; j < RB; ++j) s[j] += a * rv[j * 2 * BS + BS / 2];
+    }
+}
+
+// z = Dinv r for one right-hand side: teams of 128 threads, per step a team takes a tile of TE
+// consecutive elements, or of a large block (over 24 KB) half its entries, while the next step's are
+// copied in (cp.async): small enough stages for four teams per SM, which hide each other's
+// shared-memory latency.  Bound by the inverses' bytes: 105 x 105 FP64 blocks of 10,368 elements
+// 161 (whole square blocks, 5.7 TB/s) -> 84 us (5.5 TB/s on half the bytes); whole blocks as stages,
+// two teams per SM, 120 us; both accesses through L1 172 us.
+template <int BS, typename TM>
+struct BjacStream {
+    static constexpr int TT = 128, TE = TT / BS > 0 ? TT / BS : 1, PK = bjac_packed_size(BS), HD = BS / 2 + 1;
+    static constexpr int PARTS = (TE == 1 && PK * sizeof(TM) > 24 * 1024) ? 2 : 1;
+    static constexpr int DC = PARTS == 1 ? HD : (HD / 2 + 3) / 4 * 4;  // rows d per part: whole 16 bytes
+    static constexpr int STAGE = PARTS == 1 ? TE * PK : DC * BS;       // entries
+    static constexpr size_t smem(size_t vec) { return 2 * 2 * (STAGE * sizeof(TM) + TE * 2 * BS * vec); }
+    static_assert(PARTS == 1 || (PK - DC * BS <= STAGE && DC * BS % 4 == 0), "parts of a block");
+};
 template <int BS, typename TM, typename TV>
+__global__ void __launch_bounds__(256)
+    bjac_stream_kernel(int64_t E, const TM* __restrict__ inv, const TV* r, TV* z) {
+    using L = BjacStream<BS, TM>;
+    constexpr int TE = L::TE, TT = L::TT, PK = L::PK, PARTS = L::PARTS;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int team = threadIdx.x / TT, tid = threadIdx.x % TT;
+    TM* stage0 = reinterpret_cast<TM*>(smem_raw) + team * 2 * L::STAGE;
+    TV* vec0 = reinterpret_cast<TV*>(smem_raw + 4 * L::STAGE * sizeof(TM)) + team * 2 * (TE * 2 * BS);
+    const int64_t ntiles = (E + TE - 1) / TE, step = static_cast<int64_t>(gridDim.x) * 2;
+    const int te = tid / BS, row = tid % BS;
+    const bool mine = te < TE;
+    const auto load = [&](int64_t tile, int part, int buf) {  // these inverses on their way
+        if (tile < ntiles) {
+            const int64_t e0 = tile * TE;
+            const int entries = PARTS == 1 ? static_cast<int>(E - e0 < TE ? E - e0 : TE) * PK
+                                           : (part ? PK - L::DC * BS : L::DC * BS);
+            const char* src = reinterpret_cast<const char*>(inv + e0 * PK + part * (L::DC * BS));
+            char* dst = reinterpret_cast<char*>(stage0 + buf * L::STAGE);
+            for (int i = tid; i < entries * static_cast<int>(sizeof(TM)) / 16; i += TT) cp_async16(dst + i * 16, src + i * 16);
+        }
+        cp_async_commit();
+    };
+    const auto vec = [&](int64_t tile) {
+        const int64_t e = tile * TE + te;
+        return (mine && tile < ntiles && e < E) ? r[e * BS + row] : TV(0);
+    };
+    int64_t tile = static_cast<int64_t>(blockIdx.x) * 2 + team;
+    if (tile >= ntiles) return;  // the whole team
+    load(tile, 0, 0);
+    TV cur = vec(tile);
+    for (int k = 0; tile < ntiles; tile += step, ++k) {
+        const int64_t e = tile * TE + te;
+        const TV nxt = vec(tile + step);
+        TV* v = vec0 + (k & 1) * (TE * 2 * BS) + te * 2 * BS + row;
+        if (mine) v[0] = v[BS] = cur;
+        cur = nxt;
+        TV s[1] = {TV(0)};
+#pragma unroll
+        for (int part = 0; part < PARTS; ++part) {
+            const int buf = (k * PARTS + part) & 1;
+            load(part + 1 < PARTS ? tile : tile + step, part + 1 < PARTS ? part + 1 : 0, buf ^ 1);
+            cp_async_wait<1>();
+            mma_group_sync<TT>(team);
+            if (mine && e < E)
+                bjac_row<BS, TM, TV, 1>(stage0 + buf * L::STAGE + te * PK + row, v, row, part * L::DC,
+                                        part + 1 < PARTS ? L::DC : L::HD, s);
+            mma_group_sync<TT>(team);  // the stage is free again
+        }
+        if (mine && e < E) z[e * BS + row] = s[0];
+    }
+    cp_async_wait<0>();
+}
+
+// z = Dinv r, one thread per (element, row), RB right-hand sides at a time (blockIdx.y: the group).
+template <int BS, typename TM, typename TV, int RB>
 __global__ void __launch_bounds__(256) bjac_apply_kernel(int64_t E, const TM* __restrict__ inv,
                                                          const TV* __restrict__ r, TV* __restrict__ z,
-                                                         int64_t ld) {
-    constexpr int TE = (256 / BS) > 0 ? (256 / BS) : 1;
-    __shared__ TV sr[TE * BS];
-    const int rhs = blockIdx.y;
-    r += rhs * ld;
-    z += rhs * ld;
+                                                         int nrhs, int64_t ld) {
+    constexpr int TE = (256 / BS) > 0 ? (256 / BS) : 1, PK = bjac_packed_size(BS);
+    __shared__ TV sr[TE * RB * 2 * BS];
+    const int rhs0 = blockIdx.y * RB;
     const int64_t ntiles = (E + TE - 1) / TE;
+    const int te = threadIdx.x / BS, row = threadIdx.x % BS;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int64_t e0 = tile * TE;
+        const int64_t e0 = tile * TE, e = e0 + te;
         __syncthreads();
-        for (int i = threadIdx.x; i < TE * BS; i += blockDim.x)
-            sr[i] = (e0 + i / BS < E) ? r[e0 * BS + i] : TV(0);
+        for (int i = threadIdx.x; i < TE * RB * BS; i += blockDim.x) {
+            const int t = i / (RB * BS), j = i / BS % RB, k = i % BS;
+            const TV v = (e0 + t < E && rhs0 + j < nrhs) ? r[(rhs0 + j) * ld + (e0 + t) * BS + k] : TV(0);
+            sr[(t * RB + j) * 2 * BS + k] = v;
+            sr[(t * RB + j) * 2 * BS + BS + k] = v;
+        }
         __syncthreads();
-        const int te = threadIdx.x / BS, row = threadIdx.x % BS;
-        const int64_t e = e0 + te;
         if (te < TE && e < E) {
-            const TM* m = inv + e * BS * BS + row;
-            const TV* rv = sr + te * BS;
-            TV s = TV(0);
-#pragma unroll 8
-            for (int c = 0; c < BS; ++c) s += static_cast<TV>(m[c * BS]) * rv[c];
-            z[e * BS + row] = s;
+            TV s[RB] = {};
+            bjac_row<BS, TM, TV, RB>(inv + e * PK + row, sr + te * RB * 2 * BS + row, row, 0, BS / 2 + 1, s);
+#pragma unroll
+            for (int j = 0; j < RB; ++j)
+                if (rhs0 + j < nrhs) z[(rhs0 + j) * ld + e * BS + row] = s[j];
+        }
+    }
+}
+
+// z = Dinv r for groups of up to 8 NR FP64 right-hand sides (blockIdx.y: the group): one warp per
+// element, Z [BS x columns] = Dinv R on the FP64 tensor pipe (A: the inverse, B: the columns).  Bound
+// by the vectors' bytes (r and z may be the same): 15 x 15 blocks of 29,000 elements, 32 columns 109 -> 38 us.
+template <int BS>
+constexpr int bjac_mma_tiles() {  // n tiles a warp holds: their B fragments stay in registers
+    return BS <= 35 ? 4 : (BS <= 60 ? 2 : 1);
+}
+template <int BS, typename TM>
+__global__ void __launch_bounds__(128) bjac_mma_kernel(int64_t E, const TM* __restrict__ inv,
+                                                       const double* r, double* z, int nrhs, int64_t ld) {
+    constexpr int PK = bjac_packed_size(BS), KS = (BS + 3) / 4, MT = (BS + 7) / 8, NR = bjac_mma_tiles<BS>();
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+    const int rhs0 = blockIdx.y * 8 * NR;
+    for (int64_t e = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); e < E; e += nwarps) {
+        const TM* m = inv + e * PK;
+        double b[NR][KS];
+#pragma unroll
+        for (int n = 0; n < NR; ++n) {
+            const int c = rhs0 + n * 8 + g;
+            const double* rc = r + c * ld + e * BS;
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks) b[n][ks] = (c < nrhs && 4 * ks + t < BS) ? rc[4 * ks + t] : 0.0;
+        }
+#pragma unroll 1
+        for (int mt = 0; mt < MT; ++mt) {
+            double acc[NR][2];
+#pragma unroll
+            for (int n = 0; n < NR; ++n) acc[n][0] = acc[n][1] = 0.0;
+            const int i = mt * 8 + g;
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks) {
+                const int j = 4 * ks + t;
+                int d = j - i;
+                if (d < 0) d += BS;
+                const int at = d <= BS / 2 ? d * BS + i : (BS - d) * BS + j;
+                const double a = (i < BS && j < BS) ? static_cast<double>(m[at]) : 0.0;
+#pragma unroll
+                for (int n = 0; n < NR; ++n)
+                    if (rhs0 + n * 8 < nrhs) dmma(acc[n], a, b[n][ks]);
+            }
+#pragma unroll
+            for (int n = 0; n < NR; ++n)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int c = rhs0 + n * 8 + 2 * t + h;
+                    if (c < nrhs && i < BS) z[c * ld + e * BS + i] = acc[n][h];
+                }
         }
     }
 }
