@@ -211,6 +211,7 @@ struct MgLevel {
     double* dinv = nullptr;
     MgInterp ip{};
     double *x = nullptr, *b = nullptr, *r = nullptr, *d = nullptr, *y = nullptr, *w = nullptr;
+    double* t = nullptr;   // transposed products of the half-read level apply (levels larger than L2)
     double lmax = 0.0;
 };
 
@@ -850,6 +851,10 @@ int mg_level_apply(tdg_op* op, int l, const double* x, double* y, const double* 
         if (b) TDG_TRY(mgk(launch_vec_rsub_cols(L.n, nrhs, L.ld, b, y, s), "residual"));
         return 0;
     }
+    if (nrhs == 1 && L.t && mg_bsr_half_applies(op->h.E, mg.NB, L.bs, L.A32 ? sizeof(float) : sizeof(double))) {
+        if (L.A32) return mgk(launch_mg_bsr_half(op->h.E, mg.NB, L.bs, mg.nbr, L.A32, x, b, y, L.t, s), "level apply");
+        return mgk(launch_mg_bsr_half(op->h.E, mg.NB, L.bs, mg.nbr, L.A, x, b, y, L.t, s), "level apply");
+    }
     if (L.A32) return mgk(launch_mg_bsr_apply(op->h.E, mg.NB, L.bs, mg.nbr, L.A32, x, b, y, nrhs, L.ld, s), "level apply");
     return mgk(launch_mg_bsr_apply(op->h.E, mg.NB, L.bs, mg.nbr, L.A, x, b, y, nrhs, L.ld, s), "level apply");
 }
@@ -1022,6 +1027,9 @@ int mg_ensure_ws(tdg_op* op, int nrhs, int64_t ld, cudaStream_t s) {
         if (l + 1 < nl) {
             TDG_CUDA_TRY(mg.ws.alloc(&L.x, sz));
             TDG_CUDA_TRY(mg.ws.alloc(&L.b, sz));
+            L.t = nullptr;
+            if (mg_bsr_half_applies(op->h.E, mg.NB, L.bs, sizeof(double)))
+                TDG_CUDA_TRY(mg.ws.alloc(&L.t, static_cast<size_t>(op->h.E) * mg.NB * L.bs));
         }
         for (double** v : {&L.r, &L.d, &L.y, &L.w}) TDG_CUDA_TRY(mg.ws.alloc(v, sz));
     }

@@ -34,6 +34,13 @@ int launch_mg_triple(int64_t E, int NB, const int32_t* nbr, MgInterp ip, const d
 template <typename TA>
 int launch_mg_bsr_apply(int64_t E, int NB, int bs, const int32_t* nbr, const TA* A, const double* x,
                         const double* b, double* y, int nrhs, int64_t ld, cudaStream_t s);
+// The same for one right-hand side of a level larger than L2 (mg_bsr_half_applies), reading each
+// symmetric pair of off-diagonal blocks once: t holds E * NB * bs doubles of scratch.
+constexpr size_t kBsrHalfBytes = size_t(96) << 20;
+bool mg_bsr_half_applies(int64_t E, int NB, int bs, size_t entry);
+template <typename TA>
+int launch_mg_bsr_half(int64_t E, int NB, int bs, const int32_t* nbr, const TA* A, const double* x, const double* b,
+                       double* y, double* t, cudaStream_t s);
 // b[i] = a[i] rounded to FP32 (the mixed-precision smoother's copies of the level blocks).
 int launch_round_to_float(int64_t n, const double* a, float* b, cudaStream_t s);
 // dinv[e][i] = 1 / blocks[e * stride + i * bs + i] (point Jacobi); status set on a non-positive
