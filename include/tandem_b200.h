@@ -250,12 +250,14 @@ typedef struct {
                                residual whenever the latter has dropped by this factor
                                (0 = default: 0.1) */
     int32_t max_outer;      /* cap on reliable updates (0 = none) */
-    int32_t use_graphs;     /* capture iteration blocks in CUDA graphs (needs a non-NULL stream):
-                               each block is a device loop (a conditional while node) that ends
+    int32_t use_graphs;     /* capture iteration blocks in CUDA graphs.  On a non-NULL stream each
+                               block is a device loop (a conditional while node) that ends
                                at the iteration where a problem's recurrence residual asks for a
                                reliable update, or after 32 iterations; the host reads the
-                               scalars between blocks.  0: the host launches every iteration and
-                               checks every 8 (every one under multigrid) */
+                               scalars between blocks.  On the NULL stream (which cannot be
+                               captured) block-Jacobi blocks of 8 iterations are captured on an
+                               internal stream and replayed.  0: the host launches every iteration
+                               and checks every 8 (every one under multigrid) */
     int32_t method;         /* TDG_KSP_CG (default) or TDG_KSP_FGMRES */
     int32_t restart;        /* FGMRES restart length m (0 = 30; at most 64) */
 } tdg_solve_opts;

@@ -29,26 +29,9 @@
 
 namespace tdg {
 
-__global__ void k_dot_finalize(const double* __restrict__ partial, const int* __restrict__ seg_chunk,
-                               double* __restrict__ scal, int slot0, int slot1) {
-    const int seg = blockIdx.x;
-    double s0 = 0.0, s1 = 0.0;
-    for (int i = seg_chunk[seg] + threadIdx.x; i < seg_chunk[seg + 1]; i += blockDim.x) {
-        s0 += partial[2 * static_cast<int64_t>(i)];
-        s1 += partial[2 * static_cast<int64_t>(i) + 1];
-    }
-    __shared__ double red[2][32];
-    s0 = block_sum(s0, red[0]);
-    s1 = block_sum(s1, red[1]);
-    if (threadIdx.x == 0) {
-        if (slot0 >= 0) scal[seg * kScal + slot0] = s0;
-        if (slot1 >= 0) scal[seg * kScal + slot1] = s1;
-    }
-}
-
-__global__ void k_cg_shift(double* __restrict__ scal, int nseg, int only_replaced) {
+__global__ void k_cg_shift(double* __restrict__ scal, int nseg) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nseg && scal[r * kScal + kActive] != 0.0 && (!only_replaced || scal[r * kScal + kRepl] != 0.0))
+    if (r < nseg && scal[r * kScal + kActive] != 0.0 && scal[r * kScal + kRepl] != 0.0)
         scal[r * kScal + kRZ] = scal[r * kScal + kRZnew];
 }
 
@@ -243,6 +226,7 @@ struct MgHierarchy {
     double* scal = nullptr;
     Chunk* chunks = nullptr;
     int* seg_chunk = nullptr;
+    int* count = nullptr;  // per column, zero between kernels
     std::vector<int> seg_chunk_h;
     // the whole coarse CG (start, device loop of kCoarseBlock-iteration blocks) as one graph for
     // graph_nrhs columns of the right-hand side graph_b and the solution graph_x
@@ -765,6 +749,7 @@ struct SegPlan {
     int nseg = 0, nchunks = 0;
     const Chunk* chunks = nullptr;   // device [nchunks]
     const int* seg_chunk = nullptr;  // device [nseg + 1]
+    int* count = nullptr;            // device [nseg], zero between kernels (last_of_segment)
     // operator view of the stacked vectors: apply / precondition with nrhs and leading dimension
     int op_nrhs = 1;
     int64_t op_ld = 0;
@@ -798,8 +783,8 @@ void plan_chunks(std::vector<int64_t> const& seg_begin, std::vector<int64_t> con
 template <typename T>
 int dots(SegPlan const& sp, const T* a, const T* b, const T* c, const T* d, double* partial, double* scal, int slot0,
          int slot1, cudaStream_t s) {
-    k_dot2<T><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, a, b, c, d, partial);
-    k_dot_finalize<<<sp.nseg, 256, 0, s>>>(partial, sp.seg_chunk, scal, slot0, slot1);
+    k_dot2<T><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, a, b, c, d, partial, sp.seg_chunk, sp.count, scal, slot0,
+                                                 slot1);
     if (cudaGetLastError() != cudaSuccess) return fail(TDG_E_CUDA, "dot kernels");
     if (sp.dist) {  // one segment: sum the slots over the ranks (adjacent slots in one call)
         const bool pair = slot0 >= 0 && slot1 == slot0 + 1;
@@ -897,8 +882,7 @@ int mg_coarse_block(tdg_op* op, SegPlan const& sp, double* x, int nrhs, cudaStre
         TDG_TRY(mgk(launch_bjac_apply<double, double>(mg.cbs, mg.cnb, mg.cinv, mg.cr, mg.cz, nrhs, mg.cn, s),
                     "coarse PC"));
         TDG_TRY(dots<double>(sp, mg.cr, mg.cz, mg.cr, mg.cr, mg.partial, mg.scal, kRZnew, kRR, s));
-        k_cg_p<double><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, mg.cp, mg.cz, mg.scal);
-        k_cg_shift<<<(nrhs + 127) / 128, 128, 0, s>>>(mg.scal, nrhs);
+        k_cg_p<double><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, mg.cp, mg.cz, mg.scal, sp.seg_chunk, sp.count);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : fail(TDG_E_CUDA, "multigrid: coarse CG kernels");
 }
@@ -918,6 +902,7 @@ int mg_coarse_emit(tdg_op* op, const double* b, double* x, int nrhs, cudaStream_
     sp.nchunks = mg.seg_chunk_h[static_cast<size_t>(nrhs)];
     sp.chunks = mg.chunks;
     sp.seg_chunk = mg.seg_chunk;
+    sp.count = mg.count;
     sp.op_nrhs = nrhs;
     sp.op_ld = mg.cn;
     const size_t nc = static_cast<size_t>(mg.cn) * nrhs;
@@ -1052,6 +1037,9 @@ int mg_ensure_ws(tdg_op* op, int nrhs, int64_t ld, cudaStream_t s) {
     TDG_CUDA_TRY(mg.ws.upload(&dsc, mg.seg_chunk_h));
     mg.chunks = const_cast<Chunk*>(dch);
     mg.seg_chunk = const_cast<int*>(dsc);
+    const int* dcount = nullptr;
+    TDG_CUDA_TRY(mg.ws.upload(&dcount, std::vector<int>(static_cast<size_t>(cap), 0)));
+    mg.count = const_cast<int*>(dcount);
     TDG_CUDA_TRY(mg.ws.alloc(&mg.scal, static_cast<size_t>(cap) * kScal));
     // dot partials: the level dots (kDotBlocks + a result slot) and the coarse CG's chunk pairs
     TDG_CUDA_TRY(mg.ws.alloc(&mg.partial, std::max<size_t>(kDotBlocks + 8, 2 * hc.size())));
@@ -1914,8 +1902,7 @@ int cg_iteration(tdg_op* op, int prec, SegPlan const& sp, T* x, CgVectors<T> v, 
     TDG_TRY(precondition<T>(op, prec, v.r, v.z, sp.op_nrhs, sp.op_ld, s));
     TDG_TRY(dots<T>(sp, v.r, v.z, v.r, v.r, partial, scal, kRZnew, kRR, s));
     if (flexible) TDG_TRY(dots<T>(sp, v.z, v.q, nullptr, nullptr, partial, scal, kZQ, -1, s));
-    k_cg_p<T><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, v.p, v.z, scal, flexible ? 1 : 0);
-    k_cg_shift<<<(sp.nseg + 127) / 128, 128, 0, s>>>(scal, sp.nseg);
+    k_cg_p<T><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, v.p, v.z, scal, sp.seg_chunk, sp.count, flexible ? 1 : 0);
     return cudaGetLastError() == cudaSuccess ? 0 : fail(TDG_E_CUDA, "CG update kernels");
 }
 
@@ -2022,8 +2009,13 @@ int pcg_reliable(tdg_op* op, int prec, SegPlan const& sp, const double* b, doubl
     const bool mg = op->pc == TDG_PC_MG;
     const int kCheck = mg ? 1 : 8;
     constexpr int kBlock = 32;
+    // The legacy default stream cannot be captured: there a block of kCheck block-Jacobi iterations is
+    // captured on a side stream and replayed on s, with the host's check after every block as without
+    // graphs (10 launches of about 5 us each otherwise bound a small problem's iteration: 2D p4
+    // Poisson, 8,192 triangles, 51 us against 32 us of kernels; a multigrid iteration is long enough).
+    const bool replay = graphs && s == nullptr && !mg && !sp.dist;
     graphs = graphs && s != nullptr;
-    if (graphs) TDG_TRY(ensure_loop(op));
+    if (graphs || replay) TDG_TRY(ensure_loop(op));
     const int nseg = sp.nseg;
     if (max_updates <= 0) max_updates = 1 << 20;
     std::vector<double> tol(nseg), act(nseg), rmax(nseg), best(nseg), thr(nseg);
@@ -2078,8 +2070,26 @@ int pcg_reliable(tdg_op* op, int prec, SegPlan const& sp, const double* b, doubl
                 break;
             }
         }
+        if (replay && !exec && *iters >= kCheck) {
+            cudaStream_t cs = op->side[0];
+            cudaGraph_t graph = nullptr;
+            rc = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess ? 0 : TDG_E_CUDA;
+            for (int i = 0; i < kCheck && rc == 0; ++i) rc = cg_iteration<T>(op, prec, sp, xh, v, partial, scal, cs);
+            const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
+            if (rc == 0 && (ce != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess)) rc = TDG_E_CUDA;
+            if (graph) cudaGraphDestroy(graph);
+            if (rc) {
+                if (g_last_error.empty()) fail(rc, "capturing a CG block");
+                break;
+            }
+        }
         int done = kCheck;
-        if (exec) {
+        if (exec && replay) {
+            if (cudaGraphLaunch(exec, s) != cudaSuccess) {
+                rc = fail(TDG_E_CUDA, "graph launch");
+                break;
+            }
+        } else if (exec) {
             lc[kLoopIts] = 0;
             lc[kLoopLimit] = std::min(kBlock, max_it - *iters);
             if (cudaMemcpyAsync(op->loop, lc, sizeof lc, cudaMemcpyHostToDevice, s) != cudaSuccess ||
@@ -2098,7 +2108,7 @@ int pcg_reliable(tdg_op* op, int prec, SegPlan const& sp, const double* b, doubl
             rc = fail(TDG_E_CUDA, "reading the Krylov scalars");
             break;
         }
-        if (exec) done = static_cast<int>(lc[kLoopIts]);
+        if (exec && !replay) done = static_cast<int>(lc[kLoopIts]);
         *iters += done;
         const bool last = *iters >= max_it;
         bool update = last;
@@ -2188,7 +2198,7 @@ int pcg_reliable(tdg_op* op, int prec, SegPlan const& sp, const double* b, doubl
         if ((rc = precondition<T>(op, prec, rh, v.q, sp.op_nrhs, sp.op_ld, s))) break;
         if ((rc = dots<T>(sp, rh, v.q, rh, rh, partial, scal, kRZnew, kRR, s))) break;
         k_replace_dir<T><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, v.p, v.z, v.q, scal);
-        k_cg_shift<<<(nseg + 127) / 128, 128, 0, s>>>(scal, nseg, 1);
+        k_cg_shift<<<(nseg + 127) / 128, 128, 0, s>>>(scal, nseg);
     }
     if (exec) cudaGraphExecDestroy(exec);
     if (rc) return rc;
@@ -2343,10 +2353,10 @@ int solve_segments(tdg_op* op, const double* b, double* x, std::vector<int64_t> 
     plan_chunks(seg_begin, seg_end, hchunks, hseg);
     const int nseg = static_cast<int>(seg_begin.size());
     const size_t vec = vec_entries;
-    // every carve below is rounded up to 256 bytes: one 256-byte unit of slack per carve (9 FP64
+    // every carve below is rounded up to 256 bytes: one 256-byte unit of slack per carve (10 FP64
     // carves, 5 more for the FP32 vectors)
     size_t need = 5 * vec * sizeof(double) + hchunks.size() * (2 * sizeof(double) + sizeof(Chunk)) +
-                  (hseg.size()) * sizeof(int) + static_cast<size_t>(nseg) * kScal * sizeof(double) + 9 * 256;
+                  (hseg.size()) * sizeof(int) + static_cast<size_t>(nseg) * (kScal * sizeof(double) + sizeof(int)) + 10 * 256;
     if (prec == TDG_FP32) need += 5 * vec * sizeof(float) + 5 * 256;
     // FGMRES: V (m + 1 vectors), Z (m), w; per segment the dots, H, rotations, g, y, state; chunk
     // partials of the multi-dots (m + 2 columns)
@@ -2379,6 +2389,9 @@ int solve_segments(tdg_op* op, const double* b, double* x, std::vector<int64_t> 
     Chunk* dchunks = reinterpret_cast<Chunk*>(take(hchunks.size() * sizeof(Chunk)));
     int* dseg = reinterpret_cast<int*>(take(hseg.size() * sizeof(int)));
     double* scal = reinterpret_cast<double*>(take(static_cast<size_t>(nseg) * kScal * sizeof(double)));
+    int* count = reinterpret_cast<int*>(take(static_cast<size_t>(nseg) * sizeof(int)));
+    TDG_CUDA_TRY(cudaMemsetAsync(count, 0, static_cast<size_t>(nseg) * sizeof(int), s));
+    TDG_CUDA_TRY(cudaMemsetAsync(scal, 0, static_cast<size_t>(nseg) * kScal * sizeof(double), s));  // empty segments: 0
     TDG_CUDA_TRY(cudaMemcpyAsync(dchunks, hchunks.data(), hchunks.size() * sizeof(Chunk), cudaMemcpyHostToDevice, s));
     TDG_CUDA_TRY(cudaMemcpyAsync(dseg, hseg.data(), hseg.size() * sizeof(int), cudaMemcpyHostToDevice, s));
     SegPlan sp;
@@ -2386,6 +2399,7 @@ int solve_segments(tdg_op* op, const double* b, double* x, std::vector<int64_t> 
     sp.nchunks = static_cast<int>(hchunks.size());
     sp.chunks = dchunks;
     sp.seg_chunk = dseg;
+    sp.count = count;
     sp.op_nrhs = op_nrhs;
     sp.op_ld = op_ld;
     sp.dist = dist;

@@ -22,7 +22,9 @@ constexpr int kScal = 10;
 enum ScalSlot { kRZ = 0, kPQ = 1, kRZnew = 2, kRR = 3, kActive = 4, kBB = 5, kTmp = 6, kRepl = 7, kZQ = 8 };
 constexpr int kVecThreads = 256;
 constexpr int64_t kChunk = 32 * 1024;
-constexpr int64_t kChunkMin = 1024;
+// One entry per thread for short vectors (122,880 entries: a dot product 5.0 us with 1,024-entry chunks,
+// 120 CTAs of four dependent rounds of loads).
+constexpr int64_t kChunkMin = 256;
 
 struct Chunk {
     int64_t begin, end;  // entries [begin, end) of the stacked vector
@@ -48,11 +50,30 @@ __device__ inline double block_sum(double v, double* red) {
     return s;
 }
 
-// partial[chunk][j]: a.b (j = 0) and c.d (j = 1, when c != nullptr) over the chunk.
+// True in every thread of the CTA that finishes its segment's chunks last (count: one word per
+// segment, zero between kernels; the caller's earlier writes are visible to that CTA).
+__device__ inline bool last_of_segment(int* count, int nchunks) {
+    __shared__ int s_last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(count, 1) == nchunks - 1;
+        if (s_last) {
+            *count = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    return s_last != 0;
+}
+
+// scal[seg][slot0] = a.b and scal[seg][slot1] = c.d (when c != nullptr; slot < 0: skip): partial sums
+// per chunk, added in chunk order by the CTA that finishes its segment last, so that a dot product
+// is one launch and still deterministic.
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
     k_dot2(const Chunk* __restrict__ chunks, const T* __restrict__ a, const T* __restrict__ b,
-           const T* __restrict__ c, const T* __restrict__ d, double* __restrict__ partial) {
+           const T* __restrict__ c, const T* __restrict__ d, double* partial, const int* __restrict__ seg_chunk,
+           int* count, double* scal, int slot0, int slot1) {
     const Chunk ch = chunks[blockIdx.x];
     double s0 = 0.0, s1 = 0.0;
     for (int64_t i = ch.begin + threadIdx.x; i < ch.end; i += blockDim.x) {
@@ -66,11 +87,20 @@ __global__ void __launch_bounds__(kVecThreads)
         partial[2 * static_cast<int64_t>(blockIdx.x)] = s0;
         partial[2 * static_cast<int64_t>(blockIdx.x) + 1] = s1;
     }
+    const int c0 = seg_chunk[ch.seg], c1 = seg_chunk[ch.seg + 1];
+    if (!last_of_segment(count + ch.seg, c1 - c0)) return;
+    s0 = s1 = 0.0;
+    for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) {
+        s0 += __ldcg(partial + 2 * static_cast<int64_t>(i));
+        s1 += __ldcg(partial + 2 * static_cast<int64_t>(i) + 1);
+    }
+    s0 = block_sum(s0, red[0]);
+    s1 = block_sum(s1, red[1]);
+    if (threadIdx.x == 0) {
+        if (slot0 >= 0) scal[ch.seg * kScal + slot0] = s0;
+        if (slot1 >= 0) scal[ch.seg * kScal + slot1] = s1;
+    }
 }
-
-// scal[seg][slot_j] = sum of the chunk partials of segment seg (slot < 0: skip).
-__global__ void k_dot_finalize(const double* __restrict__ partial, const int* __restrict__ seg_chunk,
-                               double* __restrict__ scal, int slot0, int slot1);
 
 // x += alpha p, r -= alpha q with alpha = rz / pq of the segment (inactive: no-op).
 template <typename T>
@@ -91,20 +121,24 @@ __global__ void __launch_bounds__(kVecThreads)
 // p = z + beta p with beta = rz_new / rz of the segment (inactive: no-op).  flexible: beta =
 // -(z_new . q) / (p . q), the flexible CG step for a preconditioner that varies between
 // iterations (Notay, "Flexible conjugate gradients", SIAM J. Sci. Comput. 22, 2000).
+// Once the whole segment has read them, rz takes rz_new.
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
-    k_cg_p(const Chunk* __restrict__ chunks, T* __restrict__ p, const T* __restrict__ z,
-           const double* __restrict__ scal, int flexible = 0) {
+    k_cg_p(const Chunk* __restrict__ chunks, T* __restrict__ p, const T* __restrict__ z, double* scal,
+           const int* __restrict__ seg_chunk, int* count, int flexible = 0) {
     const Chunk ch = chunks[blockIdx.x];
-    const double* s = scal + ch.seg * kScal;
-    if (s[kActive] == 0.0) return;
+    double* s = scal + ch.seg * kScal;
+    if (s[kActive] == 0.0) return;  // the whole segment
     const double rz = s[kRZ], pq = s[kPQ];
     const T beta = static_cast<T>(flexible ? (pq != 0.0 ? -s[kZQ] / pq : 0.0) : (rz != 0.0 ? s[kRZnew] / rz : 0.0));
     for (int64_t i = ch.begin + threadIdx.x; i < ch.end; i += blockDim.x) p[i] = z[i] + beta * p[i];
+    __syncthreads();
+    if (last_of_segment(count + ch.seg, seg_chunk[ch.seg + 1] - seg_chunk[ch.seg]) && threadIdx.x == 0)
+        s[kRZ] = s[kRZnew];
 }
 
-// rz = rz_new for every active segment (only_replaced: for the active segments flagged kRepl).
-__global__ void k_cg_shift(double* __restrict__ scal, int nseg, int only_replaced = 0);
+// rz = rz_new for the active segments flagged kRepl.
+__global__ void k_cg_shift(double* __restrict__ scal, int nseg);
 
 // out = in on the active segments flagged kRepl (with type conversion); other segments untouched.
 template <typename Tin, typename Tout>
