@@ -173,13 +173,13 @@ int tdg_bjacobi_blocks(tdg_op* op, double* out);
 typedef struct {
     int family;       /* 0 = element-centric tensor-core kernel, 1 = SIMT kernel, 2 and 3 = face-centric
                          tensor-core kernels (volume kernel + one pass over the facets): the same
-                         warp-tile kernels in FP64 (one warp per 8 elements / facets, no barriers; 3
-                         with `tile` != 0 runs the volume term in passes), the mma.sync pair in FP32,
-                         4 = FP32 only: family 2 with the volume term on the 5th-generation tensor
+                         warp-tile kernels (one warp per 8 elements / facets, 16 in FP32; no
+                         barriers; 3 with `tile` != 0, FP64 only, runs the volume term in passes),
+                         4 = FP32 only: the volume term on the 5th-generation tensor
                          cores (tcgen05.mma kind::tf32, accumulators in tensor memory; shapes with at
                          most 64 volume points, else family 2) */
-    int ctas_per_sm;  /* persistent CTAs per SM requested (0 = default); FP64 families 2 and 3: units of
-                         4 warps of the one CTA per SM */
+    int ctas_per_sm;  /* persistent CTAs per SM requested (0 = default); warp-tile kernels: units of 4
+                         warps of the one CTA per SM */
     int tile;         /* family 3, FP64: volume quadrature points per pass of the volume kernel (its
                          GEMM tiles are D x tile rows of the volume table); 0 = the warp-tile volume
                          kernel; other families 0 */
@@ -191,7 +191,9 @@ typedef struct {
  * face-centric pair; FP32 also the pair with the tcgen05 volume kernel) at 1 to 4 persistent CTAs
  * per SM (clipped to the occupancy limit of the shape's tile), the FP64 face-centric form also at
  * the tile heights that cover the volume points in 2, 3 and 4 passes, and the SIMT kernel -- with CUDA events on
- * `stream`, and keeps the fastest for later tdg_apply / tdg_solve calls of that precision.
+ * `stream`, and keeps the fastest for later tdg_apply / tdg_solve calls of that precision.  On small
+ * shapes (2D up to 12 unknowns per element, 3D degree 1) in FP32 the SIMT kernel, the most accurate,
+ * is kept against the face-centric ones where it clearly beats the element-centric one.
  * entries (optional, up to max_entries) receives every measurement; n_entries their count. */
 int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_entry* entries, int max_entries,
                  int* n_entries);

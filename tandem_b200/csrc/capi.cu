@@ -6,8 +6,7 @@
 #include "kernels/apply_mma.cuh"
 #include "kernels/bjacobi.cuh"
 #include "kernels/apply_tc32.cuh"
-#include "kernels/apply_face.cuh"
-#include "kernels/apply_face_tc32.cuh"
+#include "kernels/apply_warp32.cuh"
 #include "kernels/apply_warp.cuh"
 #include "kernels/wave.cuh"
 #include "kernels/dispatch.hpp"
@@ -255,7 +254,7 @@ struct tdg_op {
     DevOp<float> op32;
     MmaTiles mma;           // FP64 tensor-pipe apply: packed tables and signature tiles
     Tc32Tiles tc32;         // FP32 tensor-core apply (3xTF32): packed tables and signature tiles
-    FaceTiles face32;       // face-centric FP32 apply: the same grouping with the FP32 tile size
+    WarpGeo32 warp32;       // warp-tile FP32 apply
     WarpGeo warp;           // warp-tile FP64 apply: fragment tables, lane-ordered geometry
     // explicit wave operator: basis at the volume points, reference inverse mass, -rhoInv W / |J|
     DevArena arena_wave;
@@ -402,10 +401,8 @@ void signature_tiles(HostOperator const& h, int TE, std::vector<int>& perm, std:
 // Face-centric apply: every facet with a flux once, grouped by (l0, l1, mode) -- mode 1 interior
 // (both sides), 2 boundary Dirichlet / fault (side 0), 3 boundary with code None (side 0, the
 // element as its own neighbour, as the element-centric apply treats it) -- and cut into tiles of
-// at most TE facets with one key.  finfo[f] = {up0, up1, l0 | l1 << 8, mode}.
-void facet_tiles(HostOperator const& h, int TE, std::vector<int4>& finfo, std::vector<int>& fids,
-                 std::vector<int4>& ftiles) {
-    finfo.assign(static_cast<size_t>(h.F), make_int4(0, 0, 0, 0));
+// at most TE facets with one key.
+void facet_tiles(HostOperator const& h, int TE, std::vector<int>& fids, std::vector<int4>& ftiles) {
     std::vector<int> fkey(static_cast<size_t>(h.F), 0);
     fids.clear();
     for (int64_t f = 0; f < h.F; ++f) {
@@ -421,7 +418,6 @@ void facet_tiles(HostOperator const& h, int TE, std::vector<int4>& finfo, std::v
             up1 = up0;
             l1 = l0;
         }
-        finfo[f] = make_int4(static_cast<int>(up0), static_cast<int>(up1), l0 | (l1 << 8), mode);
         if (mode) {
             fkey[f] = l0 | (l1 << 2) | (mode << 4);
             fids.push_back(static_cast<int>(f));
@@ -437,64 +433,14 @@ void facet_tiles(HostOperator const& h, int TE, std::vector<int4>& finfo, std::v
     }
 }
 
-// The facet tiles' geometry [tile][field][nq][TE] (n, n_unit, then Poisson K G0, K G1 or
-// elasticity G0, G1, lam0, mu0, lam1, mu1; unused slots zero), the penalty [tile][TE] and the facet
-// and element ids of every slot {facet, side-0 element, side-1 element (-1 unless mode 1), 0}.
-template <typename T>
-void tile_facet_geometry(HostOperator const& h, int TE, std::vector<int> const& fids, std::vector<int4> const& ftiles,
-                         std::vector<T>& fct, std::vector<double>& pen, std::vector<int4>& tids, int rows = 0,
-                         bool swizzle = false) {
-    // rows per field (>= nq, zero past nq); point q at row q, or at row face2_point(q) (an involution)
-    const int D = h.D, DD = D * D, nq = rows > 0 ? rows : h.nq, nqh = h.nq;
-    const bool poisson = h.kind == 0;
-    const int ff = 2 * D + 2 * DD + (poisson ? 0 : 4);
-    const size_t nft = ftiles.size();
-    fct.assign(nft * ff * nq * TE, T(0));
-    pen.assign(nft * TE, 0.0);
-    tids.assign(nft * TE, make_int4(-1, -1, -1, 0));
-#pragma omp parallel for schedule(static)
-    for (int64_t t = 0; t < static_cast<int64_t>(nft); ++t) {
-        const int4 td = ftiles[t];
-        const bool two = (td.z >> 4) == 1;
-        T* base = &fct[static_cast<size_t>(t) * ff * nq * TE];
-        for (int te = 0; te < td.y; ++te) {
-            const int64_t f = fids[td.x + te];
-            auto put = [&](int field, int q, double v) {
-                const int row = swizzle ? face2_point(q) : q;
-                base[(static_cast<size_t>(field) * nq + row) * TE + te] = static_cast<T>(v);
-            };
-            for (int q = 0; q < nqh; ++q) {
-                for (int i = 0; i < D; ++i) {
-                    put(i, q, h.fN[(static_cast<size_t>(f) * D + i) * nqh + q]);
-                    put(D + i, q, h.fNunit[(static_cast<size_t>(f) * D + i) * nqh + q]);
-                }
-                if (poisson) {
-                    for (int side = 0; side < 2; ++side)
-                        for (int c = 0; c < DD; ++c)
-                            put(2 * D + side * DD + c, q, h.fCoef[((static_cast<size_t>(f) * 2 + side) * DD + c) * nqh + q]);
-                } else {
-                    for (int c = 0; c < DD; ++c) {
-                        put(2 * D + c, q, h.fG0[(static_cast<size_t>(f) * DD + c) * nqh + q]);
-                        put(2 * D + DD + c, q, h.fG1[(static_cast<size_t>(f) * DD + c) * nqh + q]);
-                    }
-                    for (int c = 0; c < 4; ++c) put(2 * D + 2 * DD + c, q, h.fCoef[(static_cast<size_t>(f) * 4 + c) * nqh + q]);
-                }
-            }
-            pen[static_cast<size_t>(t) * TE + te] = h.penalty[f];
-            tids[static_cast<size_t>(t) * TE + te] = make_int4(static_cast<int>(f), static_cast<int>(h.up[2 * f]),
-                                                                two ? static_cast<int>(h.up[2 * f + 1]) : -1, 0);
-        }
-    }
-}
-
 // Tables and geometry of the warp-tile apply: facet tiles of 8 facets of one key, volume tiles of 8
 // consecutive elements.
 int upload_warp(tdg_op* op, DevArena& arena) {
     auto const& h = op->h;
     WarpGeo wg;
-    std::vector<int4> finfo, ftiles;
+    std::vector<int4> ftiles;
     std::vector<int> fids;
-    facet_tiles(h, 8, finfo, fids, ftiles);
+    facet_tiles(h, 8, fids, ftiles);
     const WarpFacetTables ft = warp_facet_tables(h);
     const int64_t nft = static_cast<int64_t>(ftiles.size()), fs = warp_facet_stride(h);
     std::vector<double> fct(static_cast<size_t>(nft) * fs, 0.0);
@@ -530,6 +476,50 @@ int upload_warp(tdg_op* op, DevArena& arena) {
     }
     wg.nftiles = static_cast<int>(nft);
     op->warp = wg;
+    return 0;
+}
+
+// The same for the FP32 kernels: tiles of 16, the penalty apart.
+int upload_warp32(tdg_op* op, DevArena& arena) {
+    auto const& h = op->h;
+    WarpGeo32 wg;
+    std::vector<int4> ftiles;
+    std::vector<int> fids;
+    facet_tiles(h, 16, fids, ftiles);
+    const WarpFacetTables32 ft = warp_facet_tables32(h);
+    const int64_t nft = static_cast<int64_t>(ftiles.size()), fs = warp_facet_stride32(h);
+    std::vector<float> fct(static_cast<size_t>(nft) * fs, 0.0f);
+    std::vector<double> pen(static_cast<size_t>(nft) * 16, 0.0);
+    std::vector<int4> tids(static_cast<size_t>(nft) * 16, make_int4(-1, -1, -1, 0));
+#pragma omp parallel for schedule(static)
+    for (int64_t t = 0; t < nft; ++t) {
+        const int4 td = ftiles[t];
+        warp_facet_tile32(h, &fids[td.x], td.y, &fct[static_cast<size_t>(t) * fs]);
+        for (int te = 0; te < td.y; ++te) {
+            const int f = fids[td.x + te];
+            pen[static_cast<size_t>(t) * 16 + te] = h.penalty[f];
+            tids[static_cast<size_t>(t) * 16 + te] =
+                make_int4(f, static_cast<int>(h.up[2 * f]), (td.z >> 4) == 1 ? static_cast<int>(h.up[2 * f + 1]) : -1, 0);
+        }
+    }
+    const int64_t nvt = (h.E + 15) / 16, vs = warp_volume_stride32(h);
+    std::vector<float> vol(static_cast<size_t>(nvt) * vs, 0.0f);
+#pragma omp parallel for schedule(static)
+    for (int64_t t = 0; t < nvt; ++t) warp_volume_tile32(h, t, &vol[static_cast<size_t>(t) * vs]);
+    if (nft) {
+        TDG_CUDA_TRY(arena.upload(&wg.fct, fct));
+        TDG_CUDA_TRY(arena.upload(&wg.pen, pen));
+        TDG_CUDA_TRY(arena.upload(&wg.ftiles, ftiles));
+        TDG_CUDA_TRY(arena.upload(&wg.tids, tids));
+    }
+    wg.face_tables = ft.tables;
+    TDG_CUDA_TRY(arena.upload(&wg.ftab, ft.frags));
+    TDG_CUDA_TRY(arena.upload(&wg.fperm, ft.perm));
+    TDG_CUDA_TRY(arena.upload(&wg.vtab, warp_volume_frags32(h)));
+    TDG_CUDA_TRY(arena.upload(&wg.vol, vol));
+    wg.status = op->tc32.status;
+    wg.nftiles = static_cast<int>(nft);
+    op->warp32 = wg;
     return 0;
 }
 
@@ -627,28 +617,10 @@ int upload_tc32(tdg_op* op, DevArena& arena) {
         TDG_CUDA_TRY(arena.upload(&st, std::vector<int>(1, 0)));
         op->tc32.status = const_cast<int*>(st);
     }
-    {
-        std::vector<int4> finfo, ftiles;
-        std::vector<int> fids;
-        facet_tiles(h, tc32_tile_elements(D, h.Q), finfo, fids, ftiles);
-        if (!fids.empty()) {
-            TDG_CUDA_TRY(arena.upload(&op->face32.fperm, fids));
-            TDG_CUDA_TRY(arena.upload(&op->face32.ftiles, ftiles));
-        }
-        TDG_CUDA_TRY(arena.upload(&op->face32.finfo, finfo));
-        op->face32.nftiles = static_cast<int>(ftiles.size());
-        std::vector<float> fct;
-        std::vector<double> pen;
-        std::vector<int4> tids;
-        // the FP32 facet kernel's point swizzle (kTc32PointSwizzle): 3D elasticity, 16-facet tiles
-        const bool swz = D == 3 && h.kind == 1 && tc32_tile_elements(D, h.Q) == 16;
-        tile_facet_geometry(h, tc32_tile_elements(D, h.Q), fids, ftiles, fct, pen, tids, swz ? (nq + 3) / 4 * 4 : nq,
-                            swz);
-        if (!ftiles.empty()) {
-            TDG_CUDA_TRY(arena.upload(&op->face32.tids, tids));
-            TDG_CUDA_TRY(arena.upload(&op->face32.geo, fct));
-            TDG_CUDA_TRY(arena.upload(&op->face32.pen, pen));
-        }
+    try {
+        TDG_TRY(upload_warp32(op, arena));
+    } catch (std::exception const& e) {
+        return fail(TDG_E_NOMEM, std::string("warp-tile tables: ") + e.what());
     }
     return 0;
 }
@@ -1528,8 +1500,8 @@ int tdg_apply(tdg_op* op, int precision, const void* x, void* y, int nrhs, int64
     const bool face32 = op->use_mma && op->family[1] >= 2;  // face-centric (the FP32 kernels have one form)
     const bool vol05 = op->family[1] == 4;                    // its volume term on tcgen05
     if (precision == TDG_FP32 && face32)
-        rc = launch_apply_face_tc32<float>(h.D, h.N, h.kind, op->op32, op->tc32, op->face32,
-                                           static_cast<const float*>(x), static_cast<float*>(y), nrhs, ld, s,
+        rc = launch_apply_warp32<float>(h.D, h.N, h.kind, op->op32, op->tc32, op->warp32,
+                                        static_cast<const float*>(x), static_cast<float*>(y), nrhs, ld, s,
                                            op->ctas[1], vol05);
     else if (precision == TDG_FP32 && tensor)
         rc = launch_apply_tc32<float>(h.D, h.N, h.kind, op->op32, op->tc32, static_cast<const float*>(x),
@@ -1540,8 +1512,8 @@ int tdg_apply(tdg_op* op, int precision, const void* x, void* y, int nrhs, int64
         // the selected tensor-core family, else the other one (a shape whose element-centric tile
         // does not fit shared memory runs face-centric, and the reverse)
         auto face = [&] {
-            return launch_apply_face_tc32<double>(h.D, h.N, h.kind, op->op32, op->tc32, op->face32,
-                                                  static_cast<const double*>(x), static_cast<double*>(y), nrhs, ld, s,
+            return launch_apply_warp32<double>(h.D, h.N, h.kind, op->op32, op->tc32, op->warp32,
+                                               static_cast<const double*>(x), static_cast<double*>(y), nrhs, ld, s,
                                                   op->ctas[1], vol05, passes);
         };
         auto elem = [&] {
@@ -1705,8 +1677,9 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    double best = 1e300;
-    int bi = -1, n = 0, rc = 0;
+    // best candidate of [0] the tile kernels (family 0), [1] the SIMT kernel, [2] the others
+    double best[3] = {1e300, 1e300, 1e300};
+    int which[3] = {-1, -1, -1}, n = 0, rc = 0;
     for (size_t i = 0; i < cands.size() && rc == 0; ++i) {
         op->family[pi] = cands[i].family;
         op->ctas[pi] = cands[i].ctas;
@@ -1727,11 +1700,23 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
         const double per = ms / reps;
         if (entries && n < max_entries) entries[n] = tdg_tune_entry{cands[i].family, cands[i].ctas, cands[i].tile, per};
         ++n;
-        if (per < best) {
-            best = per;
-            bi = static_cast<int>(i);
+        const int k = std::min(cands[i].family, 2);
+        if (per < best[k]) {
+            best[k] = per;
+            which[k] = static_cast<int>(i);
         }
     }
+    // Speed is not the only measure in FP32: the SIMT kernel sums with FMA in registers and is the
+    // most accurate (7e-8 to 1e-7 of the FP64 apply in the 2-norm against 1e-7 to 1.6e-7 of the
+    // face-centric kernels and 1.6e-7 to 2.8e-7 of family 0 below).  On the shapes where it is also
+    // clearly the faster of the two that visit elements (2D up to 12 unknowns, 3D degree 1; 16.9
+    // against 18.4 us at 2D p2 Poisson, 18,432 triangles) it therefore stays, though the face-centric
+    // kernels would take 12.5 us there.  At 2D p3 Poisson the margin is wider: it is close to both.
+    const bool small = h.D == 2 ? h.bs <= 12 : h.N == 1;
+    const bool simt = precision == TDG_FP32 && small && best[1] < (h.N <= 2 ? 0.95 : 0.8) * best[0];
+    int k = best[1] < best[0] ? 1 : 0;
+    if (!simt && best[2] < best[k]) k = 2;
+    const int bi = which[k];
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaFree(x);

@@ -28,4 +28,18 @@ void warp_volume_tile(HostOperator const& h, int64_t tile, double* out);
 int64_t warp_facet_stride(HostOperator const& h);
 void warp_facet_tile(HostOperator const& h, int const* fids, int count, double* out);
 
+// The same for the FP32 kernels (kernels/apply_warp32.cuh): tiles of 16, fragments [table][fragment]
+// [lane][2]; the facet geometry's last shared field lacks the penalty.
+struct WarpFacetTables32 {
+    std::vector<float> frags;
+    int tables = 0;
+    std::vector<int> perm;
+};
+WarpFacetTables32 warp_facet_tables32(HostOperator const& h);
+std::vector<float> warp_volume_frags32(HostOperator const& h);
+int64_t warp_facet_stride32(HostOperator const& h);
+int64_t warp_volume_stride32(HostOperator const& h);
+void warp_facet_tile32(HostOperator const& h, int const* fids, int count, float* out);
+void warp_volume_tile32(HostOperator const& h, int64_t tile, float* out);
+
 }  // namespace tdg

@@ -1,5 +1,5 @@
 // Instances and launcher of the tcgen05 volume kernel of the FP32 apply (apply_tc05.cuh).
-#include "apply_face_tc32.cuh"
+#include "apply_tc32.cuh"
 #include "apply_tc05.cuh"
 #include "dispatch.hpp"
 
@@ -34,7 +34,7 @@ int run_vol_tc05(DevOp<float> const& op, Tc32Tiles const& mt, const TX* x, TX* y
     int64_t grid = device_sm_count();  // one CTA per SM: the shared memory and half the tensor memory
     if (grid > nwork) grid = nwork;
     if (grid < 1) return 0;
-    k<<<static_cast<unsigned>(grid), kTc05Pipelined ? 512 : 256, L::BYTES, s>>>(op, mt.tables, TcfTile<S>::LDT, x, y, ld,
+    k<<<static_cast<unsigned>(grid), kTc05Pipelined ? 512 : 256, L::BYTES, s>>>(op, mt.tables, tc_round(S::NBF, 8) + 4, x, y, ld,
                                                                                  nrhs, mt.status);
     return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;
 }

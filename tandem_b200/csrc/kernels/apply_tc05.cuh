@@ -1,6 +1,6 @@
 // Volume term of the face-centric FP32 apply on the 5th-generation tensor cores (tcgen05.mma
 // kind::tf32, accumulators in tensor memory), 3xTF32 (hi hi + hi lo + lo hi, ~2^-21 per product,
-// FP32 accumulation).  It replaces vol_tc32_kernel (mma.sync) in front of face_tc32_kernel: per tile
+// FP32 accumulation).  It replaces vol_tc32_kernel (mma.sync) in front of the facet kernel: per tile
 // of TE = 16 consecutive elements it stores y = volume term (Poisson.cpp:551-575,
 // Elasticity.cpp:698-745, the same contraction and pointwise flux as the FP64 kernels).
 //
@@ -26,7 +26,7 @@
 // buffer extends past every such read.
 #pragma once
 
-#include "apply_face.cuh"
+#include "apply_tc32.cuh"
 #include "tc05.cuh"
 
 namespace tdg {

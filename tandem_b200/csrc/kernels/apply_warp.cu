@@ -1,60 +1,13 @@
 // Instances and launchers of the warp-tile FP64 apply (apply_warp.cuh).
 #include "apply_warp.cuh"
+#include "warp_plan.hpp"
 #include "dispatch.hpp"
 
 #include "../../../include/tandem_b200.h"
 
-#include <algorithm>
-
 namespace tdg {
 
 namespace {
-
-// Dynamic shared memory a CTA may take beside the kernels' static arrays.
-size_t shared_limit() {
-    static const size_t limit = [] {
-        int dev = 0, optin = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        return optin > 2048 ? static_cast<size_t>(optin) - 2048 : size_t(0);
-    }();
-    return limit;
-}
-
-// Grid, warps per CTA (one persistent CTA per SM) and split of `nwork` items of `nblk` blocks each.
-struct Plan {
-    int grid, warps;
-    WarpSplit split;
-};
-// most: warps the launch bound and shared memory allow; ctas: the caller's limit (4 warps each, 0
-// none); mma: products of an item.  A last round that fills less than 85 % of the warps is split (a
-// whole-item round of 8 warps then costs about as much as its split form: 41 k clocks at 3D p4
-// elasticity).  Items of fewer than 256 products (4 k clocks of the FP64 pipe) stay whole: their
-// time is the latency of their loads, which every part would pay again.
-Plan make_plan(int most, int64_t nwork, int nblk, int mma, int ctas) {
-    const int sms = device_sm_count();
-    Plan p;
-    if (ctas > 0) most = std::min(most, 4 * ctas);
-    if (mma < 256) nblk = 1;
-    const int64_t share = (nwork + sms - 1) / sms;  // items per SM
-    p.warps = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, share * nblk)));
-    p.grid = static_cast<int>(std::min<int64_t>(sms, nwork));
-    const int64_t all = static_cast<int64_t>(p.grid) * p.warps, rest = nwork % all;
-    p.split.whole = nwork - rest;
-    p.split.parts = std::min(nblk, p.warps);
-    if (rest * 100 >= all * 85 || p.split.parts == 1) p.split.whole = nwork + (rest ? all - rest : 0);
-    return p;
-}
-
-template <class K>
-int allow_shared(K kern, bool& ready) {
-    if (ready) return 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared_limit())) !=
-        cudaSuccess)
-        return TDG_E_CUDA;
-    ready = true;
-    return 0;
-}
 
 template <class S, bool TG>
 int launch_facets(int nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld, cudaStream_t s,
@@ -63,7 +16,7 @@ int launch_facets(int nq, WarpGeo const& wg, const double* x, double* y, int nrh
     auto kern = facew_kernel<S, TG>;
     if (int rc = allow_shared(kern, ready)) return rc;
     const int64_t nwork = static_cast<int64_t>(wg.nftiles) * nrhs;
-    Plan p = make_plan(most, nwork, WarpBlocks(nq).count(), 2 * S::Q * warp_facet_frags<S>(nq), ctas);
+    Plan p = make_plan(most, nwork, WarpBlocks(nq).count(), 2 * S::Q * warp_facet_frags<S>(nq), kSplit64, ctas);
     p.split.whole = std::min(p.split.whole, nwork);
     kern<<<p.grid, 32 * p.warps, tab + p.warps * per_warp, s>>>(nq, wg, p.split, x, y, ld, nrhs);
     return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;
@@ -90,7 +43,7 @@ int launch_volume(int64_t E, int Nq, WarpGeo const& wg, const double* x, double*
     auto kern = volw_kernel<S, TG>;
     if (int rc = allow_shared(kern, ready)) return rc;
     const int64_t nwork = (E + 7) / 8 * nrhs;
-    const Plan p = make_plan(most, nwork, WarpBlocks(Nq).count(), S::Q * warp_volume_frags<S>(Nq), ctas);
+    const Plan p = make_plan(most, nwork, WarpBlocks(Nq).count(), S::Q * warp_volume_frags<S>(Nq), kSplit64, ctas);
     const size_t smem = tab + (p.split.whole < nwork ? p.warps * per_warp : 0);
     kern<<<p.grid, 32 * p.warps, smem, s>>>(E, Nq, wg, p.split, x, y, ld, nrhs);
     return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;

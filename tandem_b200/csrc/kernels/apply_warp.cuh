@@ -31,12 +31,17 @@
 // 29,000 triangles x 32 columns 593 -> 246 us; 8,192 triangles 18.4 -> 12.8 us.  Facet atomics are
 // not on the critical path (plain stores time the same).
 //
+// Facet modes: 1 interior flux, both sides; 2 boundary (Dirichlet / fault) flux, side 0; 3 interior
+// flux of side 0 only with the element as its own neighbour (a boundary facet whose code is None, as
+// the element-centric apply treats it).  The sum over a facet's contributions is unordered
+// (atomics), so results agree with the element-centric kernels to rounding, not bit for bit.
+//
 // Tables: B fragments in the order the mma loops read them ([fragment][lane], conflict free),
 // resident in the shared memory of the persistent CTA; shapes whose tables do not fit read them
 // through L1.  Per-point geometry: the fields of 8 elements x 8 points in lane order.
 #pragma once
 
-#include "apply_face.cuh"
+#include "apply_mma.cuh"
 #include "async.cuh"
 
 #include <type_traits>

@@ -31,7 +31,6 @@ int launch_volume_warp(int D, int N, int kind, int64_t E, int Nq, WarpGeo const&
                        int nrhs, int64_t ld, cudaStream_t s, int ctas = 0);
 int launch_facets_warp(int D, int N, int kind, int nq, WarpGeo const& wg, const double* x, double* y, int nrhs,
                        int64_t ld, cudaStream_t s, int ctas = 0);
-struct FaceTiles;
 
 // The volume term in passes of qc points (apply_face2.cuh), a multiple of face2_pass_step(D);
 // TDG_E_INVALID where its buffers do not fit.
@@ -40,14 +39,14 @@ int launch_vol2(int D, int N, int kind, int64_t E, int Nq, const double* tables,
 // Granularity of qc: passes start on whole 8-row GEMM tiles.
 constexpr int face2_pass_step(int D) { return D == 3 ? 8 : 4; }
 
-// Face-centric FP32 apply (apply_face_tc32.cuh), TX = float or double vectors.
+// Face-centric FP32 apply on warp tiles (apply_warp32.cuh), TX = float or double vectors.
 struct Tc32Tiles;
-// vol05: the volume term on the 5th-generation tensor cores (apply_tc05.cuh) where the shape allows
-// it, else the mma.sync volume kernel.
+struct WarpGeo32;
+// vol05: the volume term on the 5th-generation tensor cores (apply_tc05.cuh) where the shape allows it.
 template <typename TX>
-int launch_apply_face_tc32(int D, int N, int kind, DevOp<float> const& op, Tc32Tiles const& mt, FaceTiles const& ft,
-                           const TX* x, TX* y, int nrhs, int64_t ld, cudaStream_t s, int ctas = 0, bool vol05 = false,
-                           int passes = 3);
+int launch_apply_warp32(int D, int N, int kind, DevOp<float> const& op, Tc32Tiles const& mt, WarpGeo32 const& wg,
+                        const TX* x, TX* y, int nrhs, int64_t ld, cudaStream_t s, int ctas = 0, bool vol05 = false,
+                        int passes = 3);
 // The volume term alone on the 5th-generation tensor cores (stores y); TDG_E_INVALID when the
 // shape does not fit (more than 64 volume points).
 template <typename TX>

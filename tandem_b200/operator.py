@@ -201,7 +201,7 @@ class DGOperator:
 
     def set_apply_config(self, precision: int, family: str, ctas_per_sm: int = 0, tile: int = 0) -> None:
         """Selects the apply kernel explicitly: family "tensor" (element-centric tensor cores),
-        "face" / "face2" (face-centric; the same warp-tile kernels in FP64), "tc05" (FP32:
+        "face" / "face2" (face-centric; the same warp-tile kernels), "tc05" (FP32:
         face-centric with the volume term on tcgen05) or "simt";
         ctas_per_sm 0 = the default occupancy; tile (FP64 "face2" only) = volume points per pass of
         a volume kernel in passes, a multiple of 8 (3D) or 4 (2D), 0 = the warp-tile volume kernel
