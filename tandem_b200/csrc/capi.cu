@@ -1483,14 +1483,16 @@ int tdg_apply(tdg_op* op, int precision, const void* x, void* y, int nrhs, int64
         // the warp-tile kernels; family 3 with points per pass runs the volume kernel in passes
         const double* xd = static_cast<const double*>(x);
         double* yd = static_cast<double*>(y);
-        if (op->family[0] == 3 && op->tile[0] != 0) {
+        const bool passes = op->family[0] == 3 && op->tile[0] != 0;
+        if (passes) {
             rc = launch_vol2(h.D, h.N, h.kind, h.E, h.Nq, op->mma.tables, op->warp, xd, yd, nrhs, ld, s, op->ctas[0],
                              op->tile[0]);
             if (rc == TDG_E_INVALID) return fail(rc, "points per pass do not fit this shape");
         } else {
             rc = launch_volume_warp(h.D, h.N, h.kind, h.E, h.Nq, op->warp, xd, yd, nrhs, ld, s, op->ctas[0]);
         }
-        if (rc == 0) rc = launch_facets_warp(h.D, h.N, h.kind, h.nq, op->warp, xd, yd, nrhs, ld, s, op->ctas[0]);
+        if (rc == 0) rc = launch_facets_warp(h.D, h.N, h.kind, h.nq, op->warp, xd, yd, nrhs, ld, s, op->ctas[0],
+                                              !passes);
     } else if (precision == TDG_FP64 && tensor)
         rc = launch_apply_mma(h.D, h.N, h.kind, op->op64, op->mma, static_cast<const double*>(x),
                               static_cast<double*>(y), nrhs, ld, s, op->ctas[0]);

@@ -109,6 +109,11 @@ struct WarpSplit {
     int parts = 1;  // volume: warps that share one of the split items
 };
 
+// The facet kernel may start while the volume kernel before it still runs (warp_plan.hpp): it reads x and
+// geometry at once and waits before it adds to y.
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::); }
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // The fragment tables (n doubles, even) into shared memory, ending with a barrier.  Large tables go
 // through the bulk-copy engine: one thread issues, so a CTA of few warps is not bound by its own
 // loads (110 KB at 3D p4 by one warp: 67 us); up to 8 16-byte loads per thread are quicker by hand.
@@ -487,6 +492,7 @@ __global__ void __launch_bounds__(32 * WarpTile<S>::FWARPS, 1)
     };
     const auto two_sided = [](Item const& it) { return (it.key >> 4) == 1; };
     int64_t item = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x;
+    bool waited = false;
     if (item >= nitems) return;
     Item it, nx;
     fetch(item, it);
@@ -556,6 +562,8 @@ __global__ void __launch_bounds__(32 * WarpTile<S>::FWARPS, 1)
                 b = blk.full;
                 facet_phase2<S, 1, TG>(tab + 2 * b * L::BWD, geo(One{}), side, lane, stash + b * (4 * Q * 32), yac);
             }
+            if (!waited) wait_for_previous_kernel();
+            waited = true;
             if (it.id.x >= 0) {
                 double* ye = yr + static_cast<int64_t>(side ? it.id.z : it.id.y) * BS;
 #pragma unroll
@@ -695,6 +703,7 @@ __global__ void __launch_bounds__(32 * WarpTile<S>::VWARPS, 1)
     double* sm = reinterpret_cast<double*>(smem_raw);
     double* red = sm + (TG ? 0 : frags * 32) + lane;  // partial results of the warps, at this lane
     __shared__ __align__(8) unsigned long long s_bar;
+    let_next_kernel_start();
     if constexpr (!TG) {
         if (!load_tables(sm, wg.vtab, frags * 32, &s_bar, wg.status)) return;
     }

@@ -11,11 +11,11 @@ namespace tdg {
 
 // which: 0 the volume term, 1 the facet terms; one source file per vector type and pass count
 int warp32_terms_f3(int which, int D, int N, int kind, int64_t E, int Nq, int nq, WarpGeo32 const& wg, const float* x,
-                    float* y, int nrhs, int64_t ld, cudaStream_t s, int ctas);
+                    float* y, int nrhs, int64_t ld, cudaStream_t s, int ctas, bool early);
 int warp32_terms_d3(int which, int D, int N, int kind, int64_t E, int Nq, int nq, WarpGeo32 const& wg, const double* x,
-                    double* y, int nrhs, int64_t ld, cudaStream_t s, int ctas);
+                    double* y, int nrhs, int64_t ld, cudaStream_t s, int ctas, bool early);
 int warp32_terms_d1(int which, int D, int N, int kind, int64_t E, int Nq, int nq, WarpGeo32 const& wg, const double* x,
-                    double* y, int nrhs, int64_t ld, cudaStream_t s, int ctas);
+                    double* y, int nrhs, int64_t ld, cudaStream_t s, int ctas, bool early);
 
 template <typename TX>
 int launch_apply_warp32(int D, int N, int kind, DevOp<float> const& op, Tc32Tiles const& mt, WarpGeo32 const& wg,
@@ -27,13 +27,14 @@ int launch_apply_warp32(int D, int N, int kind, DevOp<float> const& op, Tc32Tile
         rc = launch_vol_tc05<TX>(D, N, kind, op, mt, x, y, nrhs, ld, s, passes);
         if (rc && rc != TDG_E_INVALID) return rc;
     }
-    for (int which = rc == 0 ? 1 : 0; which < 2; ++which) {
+    const bool early = rc != 0;  // behind the warp-tile volume kernel
+    for (int which = early ? 0 : 1; which < 2; ++which) {
         if constexpr (std::is_same_v<TX, float>)
-            rc = warp32_terms_f3(which, D, N, kind, op.E, op.Nq, op.nq, wg, x, y, nrhs, ld, s, ctas);
+            rc = warp32_terms_f3(which, D, N, kind, op.E, op.Nq, op.nq, wg, x, y, nrhs, ld, s, ctas, early);
         else if (passes == 3)
-            rc = warp32_terms_d3(which, D, N, kind, op.E, op.Nq, op.nq, wg, x, y, nrhs, ld, s, ctas);
+            rc = warp32_terms_d3(which, D, N, kind, op.E, op.Nq, op.nq, wg, x, y, nrhs, ld, s, ctas, early);
         else
-            rc = warp32_terms_d1(which, D, N, kind, op.E, op.Nq, op.nq, wg, x, y, nrhs, ld, s, ctas);
+            rc = warp32_terms_d1(which, D, N, kind, op.E, op.Nq, op.nq, wg, x, y, nrhs, ld, s, ctas, early);
         if (rc) return rc;
     }
     return 0;

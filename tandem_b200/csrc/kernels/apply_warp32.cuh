@@ -7,9 +7,9 @@
 //
 // Bound by issue: the splits, the flux arithmetic and the products share the schedulers.  Measured on
 // a B200, FP32 vectors, against the tile products of a whole CTA behind the tcgen05 volume kernel that
-// stood here before: 3D p4 elasticity, 24,576 tetrahedra 177 us (volume 64, facets 115; before 242: 82
-// and 160); 3D p2 elasticity, 7,986 tetrahedra 23 us (39); 3D p3 Poisson, 10,368 tetrahedra 25 us (52);
-// 2D p4 Poisson, 32 right-hand sides on 9,216 triangles 162 us (502).
+// stood here before: 3D p4 elasticity, 24,576 tetrahedra 172 us (volume 64, facets 115, overlapping; before
+// 242: 82 and 160); 3D p2 elasticity, 7,986 tetrahedra 23 us (39); 3D p3 Poisson, 10,368 tetrahedra 25 us (52);
+// 2D p4 Poisson, 32 right-hand sides on 7,236 triangles 76 us (236).
 #pragma once
 
 #include "apply_tc32.cuh"
@@ -413,6 +413,7 @@ __global__ void __launch_bounds__(32 * WarpTile32<S>::WARPS, 1)
     const int nblk = blk.count();
     const int64_t nitems = sp.whole + (static_cast<int64_t>(wg.nftiles) * nrhs - sp.whole) * nblk;
     const int64_t stride = static_cast<int64_t>(nwarp) * gridDim.x;
+    bool waited = false;
     for (int64_t item = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x; item < nitems; item += stride) {
         int64_t work = item, tile, rhs;
         int b0 = 0, b1 = nblk;
@@ -481,6 +482,8 @@ __global__ void __launch_bounds__(32 * WarpTile32<S>::WARPS, 1)
                     facet32_values<S, 1, NP, TG>(tab + blk.full * L::BWD, side, lane, low != 0,
                                                  stash + blk.full * (8 * Q * 32), yac);
             }
+            if (!waited) wait_for_previous_kernel();
+            waited = true;
             TX* y0 = yr + static_cast<int64_t>(side ? id0.z : id0.y) * BS;
             TX* y1 = yr + static_cast<int64_t>(side ? id1.z : id1.y) * BS;
 #pragma unroll
@@ -627,6 +630,7 @@ __global__ void __launch_bounds__(32 * WarpTile32<S>::WARPS, 1)
     float* sm = reinterpret_cast<float*>(smem_raw);
     float* red = sm + (TG ? 0 : frags * 64) + lane;
     __shared__ __align__(8) unsigned long long s_bar;
+    let_next_kernel_start();
     if constexpr (!TG) {
         if (!load_tables(reinterpret_cast<double*>(sm), reinterpret_cast<const double*>(wg.vtab), frags * 32, &s_bar,
                          wg.status))

@@ -4,8 +4,8 @@
 namespace tdg {
 
 int warp32_terms_f3(int which, int D, int N, int kind, int64_t E, int Nq, int nq, WarpGeo32 const& wg, const float* x,
-                    float* y, int nrhs, int64_t ld, cudaStream_t s, int ctas) {
-    return warp32_terms_impl<float, 3>(which, D, N, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas);
+                    float* y, int nrhs, int64_t ld, cudaStream_t s, int ctas, bool early) {
+    return warp32_terms_impl<float, 3>(which, D, N, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas, early);
 }
 
 }  // namespace tdg

@@ -10,20 +10,21 @@ namespace tdg {
 namespace {
 
 template <class S, typename TX, int NP, bool TG>
-int go_facets(int nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs, int64_t ld, cudaStream_t s, int ctas, int most,
-              size_t tab, size_t per_warp) {
+int go_facets(int nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs, int64_t ld, cudaStream_t s, int ctas, bool early,
+              int most, size_t tab, size_t per_warp) {
     static bool ready = false;
     auto kern = facew32_kernel<S, TX, NP, TG>;
     if (int rc = allow_shared(kern, ready)) return rc;
     const int64_t nwork = static_cast<int64_t>(wg.nftiles) * nrhs;
     Plan p = make_plan(most, nwork, WarpBlocks(nq).count(), 2 * S::Q * warp32_facet_frags<S>(nq), kSplit32, ctas);
     p.split.whole = std::min(p.split.whole, nwork);
-    kern<<<p.grid, 32 * p.warps, tab + p.warps * per_warp, s>>>(nq, wg, p.split, x, y, ld, nrhs);
-    return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;
+    return launch_facet_kernel(early, kern, p.grid, 32 * p.warps, tab + p.warps * per_warp, s, nq, wg, p.split, x, y, ld,
+                               nrhs);
 }
 
 template <class S, typename TX, int NP>
-int run_facets32(int nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs, int64_t ld, cudaStream_t s, int ctas) {
+int run_facets32(int nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs, int64_t ld, cudaStream_t s, int ctas,
+                 bool early) {
     using L = WarpTile32<S>;
     if (wg.nftiles == 0) return 0;
     const size_t limit = shared_limit();
@@ -32,8 +33,8 @@ int run_facets32(int nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs, int6
     if (per_warp > limit) return TDG_E_INVALID;
     const bool fits = tab + 4 * per_warp <= limit;
     const int most = static_cast<int>(std::min<size_t>(L::WARPS, (limit - (fits ? tab : 0)) / per_warp));
-    if (fits) return go_facets<S, TX, NP, false>(nq, wg, x, y, nrhs, ld, s, ctas, most, tab, per_warp);
-    return go_facets<S, TX, NP, true>(nq, wg, x, y, nrhs, ld, s, ctas, most, 0, per_warp);
+    if (fits) return go_facets<S, TX, NP, false>(nq, wg, x, y, nrhs, ld, s, ctas, early, most, tab, per_warp);
+    return go_facets<S, TX, NP, true>(nq, wg, x, y, nrhs, ld, s, ctas, early, most, 0, per_warp);
 }
 
 template <class S, typename TX, int NP, bool TG>
@@ -66,35 +67,35 @@ int run_volume32(int64_t E, int Nq, WarpGeo32 const& wg, const TX* x, TX* y, int
 // which: 0 the volume term, 1 the facet terms
 template <class S, typename TX, int NP>
 int run32(int which, int64_t E, int Nq, int nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs, int64_t ld,
-          cudaStream_t s, int ctas) {
+          cudaStream_t s, int ctas, bool early) {
     return which == 0 ? run_volume32<S, TX, NP>(E, Nq, wg, x, y, nrhs, ld, s, ctas)
-                      : run_facets32<S, TX, NP>(nq, wg, x, y, nrhs, ld, s, ctas);
+                      : run_facets32<S, TX, NP>(nq, wg, x, y, nrhs, ld, s, ctas, early);
 }
 
 template <int D, int N, typename TX, int NP>
 int kind32(int which, int kind, int64_t E, int Nq, int nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs,
-           int64_t ld, cudaStream_t s, int ctas) {
-    if (kind == kPoisson) return run32<Shape<D, N, kPoisson>, TX, NP>(which, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas);
-    return run32<Shape<D, N, kElasticity>, TX, NP>(which, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas);
+           int64_t ld, cudaStream_t s, int ctas, bool early) {
+    if (kind == kPoisson) return run32<Shape<D, N, kPoisson>, TX, NP>(which, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas, early);
+    return run32<Shape<D, N, kElasticity>, TX, NP>(which, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas, early);
 }
 
 template <int D, typename TX, int NP>
 int deg32(int which, int N, int kind, int64_t E, int Nq, int nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs,
-          int64_t ld, cudaStream_t s, int ctas) {
+          int64_t ld, cudaStream_t s, int ctas, bool early) {
     switch (N) {
-        case 1: return kind32<D, 1, TX, NP>(which, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas);
-        case 2: return kind32<D, 2, TX, NP>(which, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas);
-        case 3: return kind32<D, 3, TX, NP>(which, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas);
-        case 4: return kind32<D, 4, TX, NP>(which, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas);
+        case 1: return kind32<D, 1, TX, NP>(which, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas, early);
+        case 2: return kind32<D, 2, TX, NP>(which, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas, early);
+        case 3: return kind32<D, 3, TX, NP>(which, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas, early);
+        case 4: return kind32<D, 4, TX, NP>(which, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas, early);
         default: return TDG_E_INVALID;
     }
 }
 
 template <typename TX, int NP>
 int warp32_terms_impl(int which, int D, int N, int kind, int64_t E, int Nq, int nq, WarpGeo32 const& wg, const TX* x, TX* y,
-          int nrhs, int64_t ld, cudaStream_t s, int ctas) {
-    if (D == 2) return deg32<2, TX, NP>(which, N, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas);
-    if (D == 3) return deg32<3, TX, NP>(which, N, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas);
+          int nrhs, int64_t ld, cudaStream_t s, int ctas, bool early) {
+    if (D == 2) return deg32<2, TX, NP>(which, N, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas, early);
+    if (D == 3) return deg32<3, TX, NP>(which, N, kind, E, Nq, nq, wg, x, y, nrhs, ld, s, ctas, early);
     return TDG_E_INVALID;
 }
 

@@ -25,12 +25,13 @@ int launch_apply_mma(int D, int N, int kind, DevOp<double> const& op, MmaTiles c
                      int nrhs, int64_t ld, cudaStream_t s, int ctas = 0);
 
 // Warp-tile FP64 apply (apply_warp.cuh): volume term (stores y) and facet terms (added into y).
-// ctas: 4 warps per SM for each (0 = as many as the shape's registers and shared memory allow).
+// ctas: 4 warps per SM for each (0 = as many as the shape's registers and shared memory allow).  early:
+// directly behind launch_volume_warp on the same x and y, so that it may start before that is done.
 struct WarpGeo;
 int launch_volume_warp(int D, int N, int kind, int64_t E, int Nq, WarpGeo const& wg, const double* x, double* y,
                        int nrhs, int64_t ld, cudaStream_t s, int ctas = 0);
 int launch_facets_warp(int D, int N, int kind, int nq, WarpGeo const& wg, const double* x, double* y, int nrhs,
-                       int64_t ld, cudaStream_t s, int ctas = 0);
+                       int64_t ld, cudaStream_t s, int ctas = 0, bool early = false);
 
 // The volume term in passes of qc points (apply_face2.cuh), a multiple of face2_pass_step(D);
 // TDG_E_INVALID where its buffers do not fit.

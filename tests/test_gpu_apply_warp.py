@@ -63,3 +63,39 @@ def test_warp_tile_apply_columns(kind, dim, n, N, nrhs):
         ref = orc.apply(X[r, :op.ndof].cpu().numpy())
         assert np.abs(Y[r, :op.ndof].cpu().numpy() - ref).max() <= 1e-12 * np.abs(ref).max()
         assert torch.all(Y[r, op.ndof:] == 7.0)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("kind,dim,n,N", [(POISSON, 2, 4, 2), (ELASTICITY, 3, 4, 2), (ELASTICITY, 3, 9, 4)])
+def test_overlapping_volume_and_facet_kernels_keep_their_order(kind, dim, n, N, captured):
+    """The facet kernel starts while the volume kernel runs.  A chain x -> A x -> A A x (each apply reads
+    what the one before it wrote, scaled by a kernel between them) gives what separate applies give."""
+    op, orc = problem(kind, dim, n, N, "tandem")
+    op.set_apply_config(FP64, "face")
+    x0 = torch.randn(op.ndof, dtype=torch.float64, device=DEV)
+    x, y = x0.clone(), torch.empty_like(x0)
+    s = torch.cuda.Stream()
+
+    def chain():
+        for _ in range(6):
+            op.apply(x, y, stream=s)
+            torch.mul(y, scale, out=x)
+
+    scale = 1.0 / np.abs(orc.apply(x0.cpu().numpy())).max()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            op.apply(x, y, stream=s)
+            s.synchronize()
+            with torch.cuda.graph(graph, stream=s):
+                chain()
+            graph.replay()
+        else:
+            chain()
+    s.synchronize()
+    ref = x0.cpu().numpy()
+    for _ in range(6):
+        ref = orc.apply(ref) * scale
+    # 1e-12 from each of the six applies, with room for what the chain makes of the first ones'
+    assert np.abs(x.cpu().numpy() - ref).max() <= 1e-10 * np.abs(ref).max()
