@@ -755,7 +755,7 @@ void plan_chunks(std::vector<int64_t> const& seg_begin, std::vector<int64_t> con
 template <typename T>
 int dots(SegPlan const& sp, const T* a, const T* b, const T* c, const T* d, double* partial, double* scal, int slot0,
          int slot1, cudaStream_t s) {
-    k_dot2<T><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, a, b, c, d, partial, sp.seg_chunk, sp.count, scal, slot0,
+    launch_early(true, k_dot2<T>, sp.nchunks, kVecThreads, 0, s, sp.chunks, a, b, c, d, partial, sp.seg_chunk, sp.count, scal, slot0,
                                                  slot1);
     if (cudaGetLastError() != cudaSuccess) return fail(TDG_E_CUDA, "dot kernels");
     if (sp.dist) {  // one segment: sum the slots over the ranks (adjacent slots in one call)
@@ -850,11 +850,12 @@ int mg_coarse_block(tdg_op* op, SegPlan const& sp, double* x, int nrhs, cudaStre
             TDG_TRY(mgk(launch_mg_bsr_apply(op->h.E, mg.NB, L.bs, mg.nbr, L.A, mg.cp, nullptr, mg.cq, nrhs, mg.cn, s),
                         "coarse A"));
         TDG_TRY(dots<double>(sp, mg.cp, mg.cq, nullptr, nullptr, mg.partial, mg.scal, kPQ, -1, s));
-        k_cg_xr<double><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, x, mg.cr, mg.cp, mg.cq, mg.scal);
+        launch_early(true, k_cg_xr<double>, sp.nchunks, kVecThreads, 0, s, sp.chunks, x, mg.cr, mg.cp, mg.cq, mg.scal);
         TDG_TRY(mgk(launch_bjac_apply<double, double>(mg.cbs, mg.cnb, mg.cinv, mg.cr, mg.cz, nrhs, mg.cn, s),
                     "coarse PC"));
         TDG_TRY(dots<double>(sp, mg.cr, mg.cz, mg.cr, mg.cr, mg.partial, mg.scal, kRZnew, kRR, s));
-        k_cg_p<double><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, mg.cp, mg.cz, mg.scal, sp.seg_chunk, sp.count);
+        launch_early(true, k_cg_p<double>, sp.nchunks, kVecThreads, 0, s, sp.chunks, mg.cp, mg.cz, mg.scal, sp.seg_chunk,
+                     sp.count, 0);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : fail(TDG_E_CUDA, "multigrid: coarse CG kernels");
 }
@@ -1885,11 +1886,11 @@ int cg_iteration(tdg_op* op, int prec, SegPlan const& sp, T* x, CgVectors<T> v, 
     const bool flexible = op->pc == TDG_PC_MG;
     TDG_TRY(krylov_apply(op, prec, sp, v.p, v.q, s));
     TDG_TRY(dots<T>(sp, v.p, v.q, nullptr, nullptr, partial, scal, kPQ, -1, s));
-    k_cg_xr<T><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, x, v.r, v.p, v.q, scal);
+    launch_early(true, k_cg_xr<T>, sp.nchunks, kVecThreads, 0, s, sp.chunks, x, v.r, v.p, v.q, scal);
     TDG_TRY(precondition<T>(op, prec, v.r, v.z, sp.op_nrhs, sp.op_ld, s));
     TDG_TRY(dots<T>(sp, v.r, v.z, v.r, v.r, partial, scal, kRZnew, kRR, s));
     if (flexible) TDG_TRY(dots<T>(sp, v.z, v.q, nullptr, nullptr, partial, scal, kZQ, -1, s));
-    k_cg_p<T><<<sp.nchunks, kVecThreads, 0, s>>>(sp.chunks, v.p, v.z, scal, sp.seg_chunk, sp.count, flexible ? 1 : 0);
+    launch_early(true, k_cg_p<T>, sp.nchunks, kVecThreads, 0, s, sp.chunks, v.p, v.z, scal, sp.seg_chunk, sp.count, flexible ? 1 : 0);
     return cudaGetLastError() == cudaSuccess ? 0 : fail(TDG_E_CUDA, "CG update kernels");
 }
 

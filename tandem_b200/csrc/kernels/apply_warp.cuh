@@ -42,6 +42,7 @@
 #pragma once
 
 #include "apply_mma.cuh"
+#include "early.cuh"
 #include "async.cuh"
 
 #include <type_traits>
@@ -108,11 +109,6 @@ struct WarpSplit {
     int64_t whole = 0;
     int parts = 1;  // volume: warps that share one of the split items
 };
-
-// The facet kernel may start while the volume kernel before it still runs (warp_plan.hpp): it reads x and
-// geometry at once and waits before it adds to y.
-__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::); }
-__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
 // The fragment tables (n doubles, even) into shared memory, ending with a barrier.  Large tables go
 // through the bulk-copy engine: one thread issues, so a CTA of few warps is not bound by its own
@@ -439,6 +435,7 @@ __global__ void __launch_bounds__(32 * WarpTile<S>::FWARPS, 1)
     __shared__ __align__(8) unsigned long long s_bar, s_gbar[L::FWARPS];
     const int tabsz = TG ? 0 : wg.face_tables * frags * 32;
     const int fstride = wg.face_tables == 1 ? 0 : frags * 32;  // between the faces' tables
+    let_next_kernel_start();
     double* gbuf = sm + tabsz + warp * facet_warp_doubles<S>(nq);
     double* stash = gbuf + (L::STREAM ? facet_side_doubles<S>(2) : 0);
     for (int i = tid; i < NF * NP; i += blockDim.x) s_perm[i] = wg.fperm[i];

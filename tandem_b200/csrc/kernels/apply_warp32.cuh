@@ -399,6 +399,7 @@ __global__ void __launch_bounds__(32 * WarpTile32<S>::WARPS, 1)
     __shared__ __align__(8) unsigned long long s_bar;
     const int tabsz = TG ? 0 : wg.face_tables * frags * 64;
     const int fstride = wg.face_tables == 1 ? 0 : frags;
+    let_next_kernel_start();
     float* stash = sm + tabsz + warp * facet32_warp_floats<S>(nq);
     for (int i = tid; i < NF * NPM; i += blockDim.x) s_perm[i] = wg.fperm[i];
     if constexpr (!TG) {

@@ -59,7 +59,7 @@ int run_rows(int64_t E, const TM* inv, const TV* r, TV* z, int nrhs, int64_t ld,
     if (grid > ntiles) grid = ntiles;
     if (grid < 1) grid = 1;
     dim3 g(static_cast<unsigned>(grid), static_cast<unsigned>((nrhs + RB - 1) / RB));
-    bjac_apply_kernel<BS, TM, TV, RB><<<g, 256, 0, s>>>(E, inv, r, z, nrhs, ld);
+    launch_early(true, bjac_apply_kernel<BS, TM, TV, RB>, g, 256, 0, s, E, inv, r, z, nrhs, ld);
     return cudaGetLastError() == cudaSuccess ? 0 : TDG_E_CUDA;
 }
 

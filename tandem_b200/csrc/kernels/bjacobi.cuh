@@ -19,6 +19,7 @@
 
 #include "apply_mma.cuh"
 #include "async.cuh"
+#include "early.cuh"
 #include "common.cuh"
 
 namespace tdg {
@@ -299,6 +300,8 @@ template <int BS, typename TM, typename TV, int RB>
 __global__ void __launch_bounds__(256) bjac_apply_kernel(int64_t E, const TM* __restrict__ inv,
                                                          const TV* __restrict__ r, TV* __restrict__ z,
                                                          int nrhs, int64_t ld) {
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     constexpr int TE = (256 / BS) > 0 ? (256 / BS) : 1, PK = bjac_packed_size(BS);
     __shared__ TV sr[TE * RB * 2 * BS];
     const int rhs0 = blockIdx.y * RB;

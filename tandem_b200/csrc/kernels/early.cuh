@@ -1,0 +1,36 @@
+// Kernels that start before the one in front of them on the stream is done (programmatic dependent
+// launch).  The front kernel calls let_next_kernel_start(); the one behind, launched with
+// launch_early, has its CTAs on the SMs when the front one ends and waits in
+// wait_for_previous_kernel() for all of its writes.  Every kernel launched this way waits in every
+// CTA that does work, before it reads anything the stream wrote or writes anything the stream reads,
+// so a chain of them stays in order.  Both calls do nothing in a plain launch.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace tdg {
+
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::); }
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+// early false: a plain launch; so is every launch into a stream capture, where the edges cost more than
+// they hide (block-Jacobi CG at 2D p4 Poisson, 8,192 triangles, replayed in blocks of 8 iterations:
+// 71.7 ms with them, 65.3 without).
+template <class... P, class... A>
+bool launch_early(bool early, void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    early = early && cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...) == cudaSuccess;
+}
+
+}  // namespace tdg

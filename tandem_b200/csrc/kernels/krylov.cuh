@@ -11,6 +11,8 @@
 // captured in a CUDA graph and replayed.
 #pragma once
 
+#include "early.cuh"
+
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -74,6 +76,8 @@ __global__ void __launch_bounds__(kVecThreads)
     k_dot2(const Chunk* __restrict__ chunks, const T* __restrict__ a, const T* __restrict__ b,
            const T* __restrict__ c, const T* __restrict__ d, double* partial, const int* __restrict__ seg_chunk,
            int* count, double* scal, int slot0, int slot1) {
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     const Chunk ch = chunks[blockIdx.x];
     double s0 = 0.0, s1 = 0.0;
     for (int64_t i = ch.begin + threadIdx.x; i < ch.end; i += blockDim.x) {
@@ -107,6 +111,8 @@ template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
     k_cg_xr(const Chunk* __restrict__ chunks, T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p,
             const T* __restrict__ q, const double* __restrict__ scal) {
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     const Chunk ch = chunks[blockIdx.x];
     const double* s = scal + ch.seg * kScal;
     if (s[kActive] == 0.0) return;
@@ -126,6 +132,8 @@ template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
     k_cg_p(const Chunk* __restrict__ chunks, T* __restrict__ p, const T* __restrict__ z, double* scal,
            const int* __restrict__ seg_chunk, int* count, int flexible = 0) {
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     const Chunk ch = chunks[blockIdx.x];
     double* s = scal + ch.seg * kScal;
     if (s[kActive] == 0.0) return;  // the whole segment

@@ -2,6 +2,7 @@
 // block-sparse kernels read the bs x bs column-major blocks with consecutive rows on consecutive
 // threads.
 #include "mg.cuh"
+#include "early.cuh"
 
 #include "../../../include/tandem_b200.h"
 
@@ -133,6 +134,7 @@ __global__ void __launch_bounds__(kT)
     k_bsr_apply_t(int64_t E, int NB, const int32_t* __restrict__ nbr, const TA* __restrict__ A,
                   const double* __restrict__ x, const double* __restrict__ b, double* __restrict__ y, int nrhs,
                   int64_t ld) {
+    let_next_kernel_start();
     const int64_t n = E * BS;
     TDG_GRID_LOOP(g, n * nrhs) {
         const int64_t c = g / n, gi = g % n;
@@ -291,6 +293,8 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_cheb_first(int64_t n, int nrhs, int64_t ld, const double* __restrict__ dinv, const double* __restrict__ r,
                  double* __restrict__ d, double* __restrict__ x, double c, int x_zero) {
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     TDG_GRID_LOOP(g, n * nrhs) {
         const int64_t j = g % n, i = (g / n) * ld + j;
         const double di = c * dinv[j] * r[i];
@@ -302,6 +306,8 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_cheb_step(int64_t n, int nrhs, int64_t ld, const double* __restrict__ dinv, const double* __restrict__ y,
                 double* __restrict__ r, double* __restrict__ d, double* __restrict__ x, double c1, double c2) {
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     TDG_GRID_LOOP(g, n * nrhs) {
         const int64_t j = g % n, i = (g / n) * ld + j;
         const double ri = r[i] - y[i];
@@ -437,6 +443,7 @@ template <int BS, typename TA>
 __global__ void __launch_bounds__(kT)
     k_bsr_half(int64_t E, int NB, const int32_t* __restrict__ nbr, const TA* __restrict__ A,
                const double* __restrict__ x, double* __restrict__ y, double* __restrict__ t) {
+    let_next_kernel_start();
     constexpr int GL = BS < 32 ? BS : 32, EPW = 32 / GL, RPL = (BS + 31) / 32, LD = BS | 1;
     constexpr int WPB = bsr_half_warps(BS);
     __shared__ double s_blk[WPB][EPW][BS * LD];
@@ -506,6 +513,8 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_bsr_gather(int64_t E, int NB, int bs, const int32_t* __restrict__ nbr, const double* __restrict__ t,
                  const double* __restrict__ b, double* __restrict__ y) {
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     TDG_GRID_LOOP(g, E * bs) {
         const int64_t e = g / bs;
         const int row = static_cast<int>(g % bs);
@@ -609,7 +618,7 @@ int launch_mg_bsr_half(int64_t E, int NB, int bs, const int32_t* nbr, const TA* 
 #undef TDG_BSR_HALF_CASE
         default: return TDG_E_INVALID;
     }
-    k_bsr_gather<<<grid_for(E * bs), kT, 0, s>>>(E, NB, bs, nbr, t, b, y);
+    launch_early(true, k_bsr_gather, grid_for(E * bs), kT, 0, s, E, NB, bs, nbr, t, b, y);
     return launched();
 }
 template int launch_mg_bsr_half<double>(int64_t, int, int, const int32_t*, const double*, const double*,
@@ -663,13 +672,13 @@ int launch_aux_prolong_add(MgAux const& a, int64_t E, const double* xc, double* 
 
 int launch_cheb_first(int64_t n, int nrhs, int64_t ld, const double* dinv, const double* r, double* d, double* x,
                       double c, int x_zero, cudaStream_t s) {
-    k_cheb_first<<<grid_for(n * nrhs), kT, 0, s>>>(n, nrhs, ld, dinv, r, d, x, c, x_zero);
+    launch_early(true, k_cheb_first, grid_for(n * nrhs), kT, 0, s, n, nrhs, ld, dinv, r, d, x, c, x_zero);
     return launched();
 }
 
 int launch_cheb_step(int64_t n, int nrhs, int64_t ld, const double* dinv, const double* y, double* r, double* d,
                      double* x, double c1, double c2, cudaStream_t s) {
-    k_cheb_step<<<grid_for(n * nrhs), kT, 0, s>>>(n, nrhs, ld, dinv, y, r, d, x, c1, c2);
+    launch_early(true, k_cheb_step, grid_for(n * nrhs), kT, 0, s, n, nrhs, ld, dinv, y, r, d, x, c1, c2);
     return launched();
 }
 

@@ -60,17 +60,7 @@ inline Plan make_plan(int most, int64_t nwork, int nblk, int mma, int least, int
 // 2D p4 elasticity, 19,886 triangles in a batch 29.8 / 28.1.
 template <class... P, class... A>
 int launch_facet_kernel(bool early, void (*kern)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3(grid);
-    c.blockDim = dim3(threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = s;
-    c.attrs = &at;
-    c.numAttrs = early ? 1 : 0;
-    return cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...) == cudaSuccess ? 0 : TDG_E_CUDA;
+    return launch_early(early, kern, dim3(grid), threads, smem, s, args...) ? 0 : TDG_E_CUDA;
 }
 
 template <class K>
