@@ -755,8 +755,8 @@ void plan_chunks(std::vector<int64_t> const& seg_begin, std::vector<int64_t> con
 template <typename T>
 int dots(SegPlan const& sp, const T* a, const T* b, const T* c, const T* d, double* partial, double* scal, int slot0,
          int slot1, cudaStream_t s) {
-    launch_early(true, k_dot2<T>, sp.nchunks, kVecThreads, 0, s, sp.chunks, a, b, c, d, partial, sp.seg_chunk, sp.count, scal, slot0,
-                                                 slot1);
+    launch_early(true, k_dot2<T>, sp.nchunks, kVecThreads, 0, s, sp.chunks, a, b, c, d, partial, sp.seg_chunk, sp.count,
+                 scal, slot0, slot1);
     if (cudaGetLastError() != cudaSuccess) return fail(TDG_E_CUDA, "dot kernels");
     if (sp.dist) {  // one segment: sum the slots over the ranks (adjacent slots in one call)
         const bool pair = slot0 >= 0 && slot1 == slot0 + 1;
@@ -1890,7 +1890,8 @@ int cg_iteration(tdg_op* op, int prec, SegPlan const& sp, T* x, CgVectors<T> v, 
     TDG_TRY(precondition<T>(op, prec, v.r, v.z, sp.op_nrhs, sp.op_ld, s));
     TDG_TRY(dots<T>(sp, v.r, v.z, v.r, v.r, partial, scal, kRZnew, kRR, s));
     if (flexible) TDG_TRY(dots<T>(sp, v.z, v.q, nullptr, nullptr, partial, scal, kZQ, -1, s));
-    launch_early(true, k_cg_p<T>, sp.nchunks, kVecThreads, 0, s, sp.chunks, v.p, v.z, scal, sp.seg_chunk, sp.count, flexible ? 1 : 0);
+    launch_early(true, k_cg_p<T>, sp.nchunks, kVecThreads, 0, s, sp.chunks, v.p, v.z, scal, sp.seg_chunk, sp.count,
+                 flexible ? 1 : 0);
     return cudaGetLastError() == cudaSuccess ? 0 : fail(TDG_E_CUDA, "CG update kernels");
 }
 

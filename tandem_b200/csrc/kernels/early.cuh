@@ -1,9 +1,11 @@
 // Kernels that start before the one in front of them on the stream is done (programmatic dependent
 // launch).  The front kernel calls let_next_kernel_start(); the one behind, launched with
 // launch_early, has its CTAs on the SMs when the front one ends and waits in
-// wait_for_previous_kernel() for all of its writes.  Every kernel launched this way waits in every
-// CTA that does work, before it reads anything the stream wrote or writes anything the stream reads,
-// so a chain of them stays in order.  Both calls do nothing in a plain launch.
+// wait_for_previous_kernel() until all of its writes are visible.  A chain stays in order because
+// every warp that works waits: the vector kernels first of all, the facet kernel before it touches
+// y.  What the facet kernel reads before that (x, geometry) the volume kernel in front of it does
+// not write, and that one is launched plainly, so whatever wrote x is done when it starts.  Both
+// calls do nothing in a plain launch.
 #pragma once
 
 #include <cuda_runtime.h>

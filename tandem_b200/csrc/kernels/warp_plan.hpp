@@ -3,6 +3,7 @@
 
 #include "apply_warp.cuh"
 #include "dispatch.hpp"
+#include "early.cuh"
 
 #include "../../../include/tandem_b200.h"
 
