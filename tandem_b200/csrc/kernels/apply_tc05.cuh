@@ -1,6 +1,6 @@
 // Volume term of the face-centric FP32 apply on the 5th-generation tensor cores (tcgen05.mma
 // kind::tf32, accumulators in tensor memory), 3xTF32 (hi hi + hi lo + lo hi, ~2^-21 per product,
-// FP32 accumulation).  It replaces vol_tc32_kernel (mma.sync) in front of the facet kernel: per tile
+// FP32 accumulation).  It runs in front of the facet kernel of apply_warp32.cuh: per tile
 // of TE = 16 consecutive elements it stores y = volume term (Poisson.cpp:551-575,
 // Elasticity.cpp:698-745, the same contraction and pointwise flux as the FP64 kernels).
 //
@@ -78,7 +78,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Pointwise volume flux at one point of one element (the same arithmetic as vol_tc32_kernel):
+// Pointwise volume flux at one point of one element (the arithmetic of the mma.sync kernels):
 // g[a][r] = d u_r / d xi_a in, T[a][r] (the lifted flux) out.
 template <class S>
 __device__ __forceinline__ void vol_point(const float (&G)[S::DD], float c0, float c1, const float (&g)[S::D][S::Q],
