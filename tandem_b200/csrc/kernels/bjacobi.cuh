@@ -327,21 +327,28 @@ __global__ void __launch_bounds__(256) bjac_apply_kernel(int64_t E, const TM* __
     }
 }
 
-// z = Dinv r for groups of up to 8 NR FP64 right-hand sides (blockIdx.y: the group): one warp per
-// element, Z [BS x columns] = Dinv R on the FP64 tensor pipe (A: the inverse, B: the columns).  Bound
-// by the vectors' bytes (r and z may be the same): 15 x 15 blocks of 29,000 elements, 32 columns 109 -> 38 us.
+// z = Dinv r for groups of up to 8 NR FP64 right-hand sides (blockIdx.y: the group), Z [BS x columns] =
+// Dinv R on the FP64 tensor pipe (A: the inverse, B: the columns).  Bound by the vectors' bytes (r and z may be
+// the same): 15 x 15 blocks of 17,712 elements, 32 columns 109 -> 38 us.  W warps share the row tiles of an
+// element: one for small blocks; four from 60, where one warp's chain of (BS / 8)(BS / 4) loads and
+// products is the time (105 x 105, 6,000 elements, 8 columns: 272 us with one warp, 112 with four; 48
+// elements 50 and 8.6).
 template <int BS>
 constexpr int bjac_mma_tiles() {  // n tiles a warp holds: their B fragments stay in registers
     return BS <= 35 ? 4 : (BS <= 60 ? 2 : 1);
+}
+template <int BS>
+constexpr int bjac_mma_warps() {
+    return BS < 60 ? 1 : 4;
 }
 template <int BS, typename TM>
 __global__ void __launch_bounds__(128) bjac_mma_kernel(int64_t E, const TM* __restrict__ inv,
                                                        const double* r, double* z, int nrhs, int64_t ld) {
     constexpr int PK = bjac_packed_size(BS), KS = (BS + 3) / 4, MT = (BS + 7) / 8, NR = bjac_mma_tiles<BS>();
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+    constexpr int W = bjac_mma_warps<BS>(), EPC = 4 / W;  // elements of a CTA
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int rhs0 = blockIdx.y * 8 * NR;
-    for (int64_t e = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); e < E; e += nwarps) {
+    for (int64_t e = static_cast<int64_t>(blockIdx.x) * EPC + warp / W; e < E; e += static_cast<int64_t>(gridDim.x) * EPC) {
         const TM* m = inv + e * PK;
         double b[NR][KS];
 #pragma unroll
@@ -351,8 +358,9 @@ __global__ void __launch_bounds__(128) bjac_mma_kernel(int64_t E, const TM* __re
 #pragma unroll
             for (int ks = 0; ks < KS; ++ks) b[n][ks] = (c < nrhs && 4 * ks + t < BS) ? rc[4 * ks + t] : 0.0;
         }
+        if constexpr (W > 1) __syncthreads();  // in place: every warp has read the element's rows
 #pragma unroll 1
-        for (int mt = 0; mt < MT; ++mt) {
+        for (int mt = warp % W; mt < MT; mt += W) {
             double acc[NR][2];
 #pragma unroll
             for (int n = 0; n < NR; ++n) acc[n][0] = acc[n][1] = 0.0;
