@@ -15,13 +15,10 @@ namespace tdg {
 __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::); }
 __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
-// early false: a plain launch; so is every launch into a stream capture, where the edges cost more than
-// they hide (block-Jacobi CG at 2D p4 Poisson, 8,192 triangles, replayed in blocks of 8 iterations:
-// 71.7 ms with them, 65.3 without).
+// early false: a plain launch.
 template <class... P, class... A>
-bool launch_early(bool early, void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    early = early && cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+bool launch_programmatic(bool early, void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s,
+                         A... args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -33,6 +30,16 @@ bool launch_early(bool early, void (*kern)(P...), dim3 grid, int threads, size_t
     c.attrs = &at;
     c.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...) == cudaSuccess;
+}
+
+// The short solver kernels, whose launches into a stream capture are plain: with an edge at every kernel of
+// a CG iteration the edges cost more than they hide (block-Jacobi CG at 2D p4 Poisson, 8,192 triangles,
+// replayed in blocks of 8 iterations: 71.7 ms with them, 65.3 without).
+template <class... P, class... A>
+bool launch_early(bool early, void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    early = early && cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    return launch_programmatic(early, kern, grid, threads, smem, s, args...);
 }
 
 }  // namespace tdg

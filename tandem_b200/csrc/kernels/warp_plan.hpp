@@ -58,10 +58,12 @@ inline Plan make_plan(int most, int64_t nwork, int nblk, int mma, int least, int
 // (launch, tables, coefficients, geometry, products), which the two kernels then share; large ones
 // fill the tail of the volume kernel.  FP64 apply without / with it, us: 3D p4 elasticity 162 tetrahedra
 // 23.1 / 14.3, 48,000 368 / 364; 3D p2 elasticity 7,986 29.7 / 26.3; 3D p3 Poisson 13,182 34.8 / 31.8;
-// 2D p4 elasticity, 19,886 triangles in a batch 29.8 / 28.1.
+// 2D p4 elasticity, 19,886 triangles in a batch 29.8 / 28.1.  Under capture too, per apply of a replayed
+// chain: 3D p2 elasticity, 162 tetrahedra 14.1 / 9.6, p4 21.8 / 14.7; 2D p4 Poisson, 8,192 triangles 9.3 / 8.4;
+// block-Jacobi CG in replayed blocks, 3D p2 elasticity, 162 tetrahedra 11.8 / 10.1 ms, p4 29.6 / 25.0.
 template <class... P, class... A>
 int launch_facet_kernel(bool early, void (*kern)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
-    return launch_early(early, kern, dim3(grid), threads, smem, s, args...) ? 0 : TDG_E_CUDA;
+    return launch_programmatic(early, kern, dim3(grid), threads, smem, s, args...) ? 0 : TDG_E_CUDA;
 }
 
 template <class K>
