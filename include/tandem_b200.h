@@ -200,6 +200,14 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
 /* Sets the apply configuration of `precision` (TDG_FP64 / TDG_FP32; TDG_MIXED and TDG_TF32 follow TDG_FP32)
  * explicitly: kernel family as in tdg_tune_entry and persistent CTAs per SM. */
 int tdg_set_apply_config(tdg_op* op, int precision, int family, int ctas_per_sm);
+/* Another configuration for tdg_apply calls alone, for a caller that needs longer to issue a call than the
+ * device needs to run it (one launch may then be quicker than two shorter ones): family -1 takes it back.
+ * Solves, preconditioners, tdg_apply_host and applies into a stream capture never use it; tdg_autotune,
+ * tdg_set_apply_config and tdg_set_apply_tile take it back. */
+int tdg_set_call_config(tdg_op* op, int precision, int family, int ctas_per_sm);
+/* The configuration that applies and solves use now (any of the outputs may be NULL): what
+ * tdg_autotune kept, tdg_set_apply_config / tdg_set_apply_tile set, or the default. */
+int tdg_get_apply_config(const tdg_op* op, int precision, int* family, int* ctas_per_sm, int* tile);
 /* Sets the tile height of family 3 (TDG_FP64 only): volume points per pass of its volume kernel, as
  * tdg_tune_entry.tile; a multiple of 8 (3D) or 4 (2D), or 0 for the warp-tile volume kernel.  A height whose
  * buffers do not fit the shape makes tdg_apply return TDG_E_INVALID. */

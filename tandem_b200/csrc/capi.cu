@@ -266,6 +266,9 @@ struct tdg_op {
     // per SM (0 = default); set by tdg_autotune
     int family[2] = {0, 0};
     int ctas[2] = {0, 0};
+    // of single tdg_apply calls, where they differ (-1: they do not)
+    int call_family[2] = {-1, -1};
+    int call_ctas[2] = {0, 0};
     // volume points per pass of the FP64 face-centric pipelined volume kernel (0 = automatic)
     int tile[2] = {0, 0};
     const double* penalty = nullptr;
@@ -770,12 +773,80 @@ int dots(SegPlan const& sp, const T* a, const T* b, const T* c, const T* d, doub
     return 0;
 }
 
+// y = A x with the operator's configuration; call: with the one set for single calls (tdg_set_call_config).
+int apply_as(tdg_op* op, int precision, const void* x, void* y, int nrhs, int64_t ld, cudaStream_t s,
+             bool call = false) {
+    if (!op || !x || !y) return fail(TDG_E_INVALID, "null argument");
+    auto const& h = op->h;
+    if (nrhs < 1 || ld < h.E * h.bs) return fail(TDG_E_INVALID, "nrhs < 1 or ld < E * bs");
+    if (x == y) return fail(TDG_E_INVALID, "x and y must not alias");
+    TDG_TRY(ensure_uploaded(op, precision));
+    int rc = TDG_E_INVALID;
+    const int pi = precision == TDG_FP64 ? 0 : 1;
+    const int family = call ? op->call_family[pi] : op->family[pi], ctas = call ? op->call_ctas[pi] : op->ctas[pi];
+    const int tile = call ? 0 : op->tile[pi];
+    const bool tensor = op->use_mma && family == 0;
+    if (precision == TDG_FP64 && op->use_mma && family >= 2) {
+        // the warp-tile kernels; family 3 with points per pass runs the volume kernel in passes
+        const double* xd = static_cast<const double*>(x);
+        double* yd = static_cast<double*>(y);
+        const bool passes = family == 3 && tile != 0;
+        if (passes) {
+            rc = launch_vol2(h.D, h.N, h.kind, h.E, h.Nq, op->mma.tables, op->warp, xd, yd, nrhs, ld, s, ctas,
+                             tile);
+            if (rc == TDG_E_INVALID) return fail(rc, "points per pass do not fit this shape");
+        } else {
+            rc = launch_volume_warp(h.D, h.N, h.kind, h.E, h.Nq, op->warp, xd, yd, nrhs, ld, s, ctas);
+        }
+        if (rc == 0) rc = launch_facets_warp(h.D, h.N, h.kind, h.nq, op->warp, xd, yd, nrhs, ld, s, ctas,
+                                              !passes);
+    } else if (precision == TDG_FP64 && tensor)
+        rc = launch_apply_mma(h.D, h.N, h.kind, op->op64, op->mma, static_cast<const double*>(x),
+                              static_cast<double*>(y), nrhs, ld, s, ctas);
+    if (precision == TDG_FP64 && rc == TDG_E_INVALID)
+        rc = launch_apply<double>(h.D, h.N, h.kind, op->op64, static_cast<const double*>(x),
+                                  static_cast<double*>(y), nrhs, ld, s);
+    const bool face32 = op->use_mma && family >= 2;  // face-centric (the FP32 kernels have one form)
+    const bool vol05 = family == 4;                    // its volume term on tcgen05
+    if (precision == TDG_FP32 && face32)
+        rc = launch_apply_warp32<float>(h.D, h.N, h.kind, op->op32, op->tc32, op->warp32,
+                                        static_cast<const float*>(x), static_cast<float*>(y), nrhs, ld, s,
+                                           ctas, vol05);
+    else if (precision == TDG_FP32 && tensor)
+        rc = launch_apply_tc32<float>(h.D, h.N, h.kind, op->op32, op->tc32, static_cast<const float*>(x),
+                                      static_cast<float*>(y), nrhs, ld, s, ctas);
+    if (precision == TDG_MIXED || precision == TDG_TF32) {
+        if (!op->use_mma) return fail(TDG_E_INVALID, "TDG_MIXED / TDG_TF32 need the tensor-core kernels");
+        const int passes = precision == TDG_TF32 ? 1 : 3;  // one TF32 pass, or 3xTF32
+        // the selected tensor-core family, else the other one (a shape whose element-centric tile
+        // does not fit shared memory runs face-centric, and the reverse)
+        auto face = [&] {
+            return launch_apply_warp32<double>(h.D, h.N, h.kind, op->op32, op->tc32, op->warp32,
+                                               static_cast<const double*>(x), static_cast<double*>(y), nrhs, ld, s,
+                                                  ctas, vol05, passes);
+        };
+        auto elem = [&] {
+            return launch_apply_tc32<double>(h.D, h.N, h.kind, op->op32, op->tc32, static_cast<const double*>(x),
+                                             static_cast<double*>(y), nrhs, ld, s, ctas, passes);
+        };
+        rc = face32 ? face() : elem();
+        if (rc == TDG_E_INVALID) rc = face32 ? elem() : face();
+        if (rc) return fail(rc, std::string("mixed apply launch failed: ") + cudaGetErrorString(cudaGetLastError()));
+        return 0;
+    }
+    if (precision == TDG_FP32 && rc == TDG_E_INVALID)
+        rc = launch_apply<float>(h.D, h.N, h.kind, op->op32, static_cast<const float*>(x),
+                                 static_cast<float*>(y), nrhs, ld, s);
+    if (rc) return fail(rc, std::string("apply launch failed: ") + cudaGetErrorString(cudaGetLastError()));
+    return 0;
+}
+
 // The apply of the Krylov drivers: y = A x, with the ghost exchange of x in front for a
 // distributed solve.
 int krylov_apply(tdg_op* op, int prec, SegPlan const& sp, void* x, void* y, cudaStream_t s) {
     if (sp.dist && sp.dist->exchange(sp.dist->ctx, static_cast<double*>(x), s) != 0)
         return fail(TDG_E_STATE, "the exchange callback of the distributed solve failed");
-    return tdg_apply(op, prec, x, y, sp.op_nrhs, sp.op_ld, s);
+    return apply_as(op, prec, x, y, sp.op_nrhs, sp.op_ld, s);
 }
 
 // ---- block-Jacobi diagonal blocks ---------------------------------------------------------------
@@ -805,7 +876,7 @@ int mg_level_apply(tdg_op* op, int l, const double* x, double* y, const double* 
     auto& mg = op->mg;
     auto const& L = mg.lv[static_cast<size_t>(l)];
     if (l + 1 == static_cast<int>(mg.lv.size())) {
-        TDG_TRY(tdg_apply(op, mg.fine_prec, x, y, nrhs, L.ld, s));
+        TDG_TRY(apply_as(op, mg.fine_prec, x, y, nrhs, L.ld, s));
         if (b) TDG_TRY(mgk(launch_vec_rsub_cols(L.n, nrhs, L.ld, b, y, s), "residual"));
         return 0;
     }
@@ -1124,7 +1195,7 @@ int mg_probe(tdg_op* op, cudaStream_t s) {
             const int nb = std::min(nj, C.bs - j0);
             if (cudaMemsetAsync(V, 0, sizeof(double) * nb * nf, s) != cudaSuccess) rc = fail(TDG_E_CUDA, "memset");
             if (!rc) rc = mgk(launch_mg_probe_fill(E, mg.colour, c, C.ip, j0, nb, V, nf, s), "probe fill");
-            if (!rc) rc = tdg_apply(op, TDG_FP64, V, Y, nb, nf, s);
+            if (!rc) rc = apply_as(op, TDG_FP64, V, Y, nb, nf, s);
             if (!rc)
                 rc = mgk(launch_mg_probe_extract(E, mg.NB, mg.nbr, mg.colour, c, C.ip, j0, nb, Y, nf, C.A, s),
                          "probe extract");
@@ -1472,68 +1543,10 @@ int tdg_penalty(const tdg_op* op, double* out) {
 }
 
 int tdg_apply(tdg_op* op, int precision, const void* x, void* y, int nrhs, int64_t ld, void* stream) {
-    if (!op || !x || !y) return fail(TDG_E_INVALID, "null argument");
-    auto const& h = op->h;
-    if (nrhs < 1 || ld < h.E * h.bs) return fail(TDG_E_INVALID, "nrhs < 1 or ld < E * bs");
-    if (x == y) return fail(TDG_E_INVALID, "x and y must not alias");
-    TDG_TRY(ensure_uploaded(op, precision));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int rc = TDG_E_INVALID;
-    const int pi = precision == TDG_FP64 ? 0 : 1;
-    const bool tensor = op->use_mma && op->family[pi] == 0;
-    if (precision == TDG_FP64 && op->use_mma && op->family[0] >= 2) {
-        // the warp-tile kernels; family 3 with points per pass runs the volume kernel in passes
-        const double* xd = static_cast<const double*>(x);
-        double* yd = static_cast<double*>(y);
-        const bool passes = op->family[0] == 3 && op->tile[0] != 0;
-        if (passes) {
-            rc = launch_vol2(h.D, h.N, h.kind, h.E, h.Nq, op->mma.tables, op->warp, xd, yd, nrhs, ld, s, op->ctas[0],
-                             op->tile[0]);
-            if (rc == TDG_E_INVALID) return fail(rc, "points per pass do not fit this shape");
-        } else {
-            rc = launch_volume_warp(h.D, h.N, h.kind, h.E, h.Nq, op->warp, xd, yd, nrhs, ld, s, op->ctas[0]);
-        }
-        if (rc == 0) rc = launch_facets_warp(h.D, h.N, h.kind, h.nq, op->warp, xd, yd, nrhs, ld, s, op->ctas[0],
-                                              !passes);
-    } else if (precision == TDG_FP64 && tensor)
-        rc = launch_apply_mma(h.D, h.N, h.kind, op->op64, op->mma, static_cast<const double*>(x),
-                              static_cast<double*>(y), nrhs, ld, s, op->ctas[0]);
-    if (precision == TDG_FP64 && rc == TDG_E_INVALID)
-        rc = launch_apply<double>(h.D, h.N, h.kind, op->op64, static_cast<const double*>(x),
-                                  static_cast<double*>(y), nrhs, ld, s);
-    const bool face32 = op->use_mma && op->family[1] >= 2;  // face-centric (the FP32 kernels have one form)
-    const bool vol05 = op->family[1] == 4;                    // its volume term on tcgen05
-    if (precision == TDG_FP32 && face32)
-        rc = launch_apply_warp32<float>(h.D, h.N, h.kind, op->op32, op->tc32, op->warp32,
-                                        static_cast<const float*>(x), static_cast<float*>(y), nrhs, ld, s,
-                                           op->ctas[1], vol05);
-    else if (precision == TDG_FP32 && tensor)
-        rc = launch_apply_tc32<float>(h.D, h.N, h.kind, op->op32, op->tc32, static_cast<const float*>(x),
-                                      static_cast<float*>(y), nrhs, ld, s, op->ctas[1]);
-    if (precision == TDG_MIXED || precision == TDG_TF32) {
-        if (!op->use_mma) return fail(TDG_E_INVALID, "TDG_MIXED / TDG_TF32 need the tensor-core kernels");
-        const int passes = precision == TDG_TF32 ? 1 : 3;  // one TF32 pass, or 3xTF32
-        // the selected tensor-core family, else the other one (a shape whose element-centric tile
-        // does not fit shared memory runs face-centric, and the reverse)
-        auto face = [&] {
-            return launch_apply_warp32<double>(h.D, h.N, h.kind, op->op32, op->tc32, op->warp32,
-                                               static_cast<const double*>(x), static_cast<double*>(y), nrhs, ld, s,
-                                                  op->ctas[1], vol05, passes);
-        };
-        auto elem = [&] {
-            return launch_apply_tc32<double>(h.D, h.N, h.kind, op->op32, op->tc32, static_cast<const double*>(x),
-                                             static_cast<double*>(y), nrhs, ld, s, op->ctas[1], passes);
-        };
-        rc = face32 ? face() : elem();
-        if (rc == TDG_E_INVALID) rc = face32 ? elem() : face();
-        if (rc) return fail(rc, std::string("mixed apply launch failed: ") + cudaGetErrorString(cudaGetLastError()));
-        return 0;
-    }
-    if (precision == TDG_FP32 && rc == TDG_E_INVALID)
-        rc = launch_apply<float>(h.D, h.N, h.kind, op->op32, static_cast<const float*>(x),
-                                 static_cast<float*>(y), nrhs, ld, s);
-    if (rc) return fail(rc, std::string("apply launch failed: ") + cudaGetErrorString(cudaGetLastError()));
-    return 0;
+    const int pi = precision == TDG_FP64 ? 0 : (precision == TDG_FP32 ? 1 : -1);
+    const bool call = op && pi >= 0 && op->call_family[pi] >= 0 && !capturing(s);
+    return apply_as(op, precision, x, y, nrhs, ld, s, call);
 }
 
 int tdg_apply_host(tdg_op* op, int precision, const void* x_host, void* y_host, int count, int64_t host_stride,
@@ -1590,7 +1603,7 @@ int tdg_apply_host(tdg_op* op, int precision, const void* x_host, void* y_host, 
         TDG_CUDA_TRY(cudaEventRecord(hs.in[b], cin));
         TDG_CUDA_TRY(cudaStreamWaitEvent(cmp, hs.in[b], 0));
         if (i >= 2) TDG_CUDA_TRY(cudaStreamWaitEvent(cmp, hs.freed[b], 0));
-        TDG_TRY(tdg_apply(op, precision, hs.xd[b], hs.yd[b], 1, n, cmp));
+        TDG_TRY(apply_as(op, precision, hs.xd[b], hs.yd[b], 1, n, cmp));
         TDG_CUDA_TRY(cudaEventRecord(hs.out[b], cmp));
         TDG_CUDA_TRY(cudaStreamWaitEvent(cout, hs.out[b], 0));
         TDG_CUDA_TRY(cudaMemcpyAsync(yb + i * hstep, hs.yd[b], bytes, cudaMemcpyDeviceToHost, cout));
@@ -1619,6 +1632,26 @@ int tdg_set_apply_config(tdg_op* op, int precision, int family, int ctas_per_sm)
     const int pi = precision == TDG_FP64 ? 0 : 1;
     op->family[pi] = family;
     op->ctas[pi] = ctas_per_sm;
+    op->call_family[pi] = -1;
+    return 0;
+}
+
+int tdg_set_call_config(tdg_op* op, int precision, int family, int ctas_per_sm) {
+    if (!op || (precision != TDG_FP64 && precision != TDG_FP32) || family < -1 || family > 4 || ctas_per_sm < 0 ||
+        (family == 4 && precision != TDG_FP32))
+        return fail(TDG_E_INVALID, "bad argument");
+    const int pi = precision == TDG_FP64 ? 0 : 1;
+    op->call_family[pi] = family;
+    op->call_ctas[pi] = ctas_per_sm;
+    return 0;
+}
+
+int tdg_get_apply_config(const tdg_op* op, int precision, int* family, int* ctas_per_sm, int* tile) {
+    if (!op || (precision != TDG_FP64 && precision != TDG_FP32)) return fail(TDG_E_INVALID, "bad argument");
+    const int pi = precision == TDG_FP64 ? 0 : 1;
+    if (family) *family = op->family[pi];
+    if (ctas_per_sm) *ctas_per_sm = op->ctas[pi];
+    if (tile) *tile = op->tile[pi];
     return 0;
 }
 
@@ -1627,7 +1660,9 @@ int tdg_set_apply_tile(tdg_op* op, int precision, int points_per_pass) {
         return fail(TDG_E_INVALID, "bad argument");
     if (points_per_pass != 0 && (precision != TDG_FP64 || points_per_pass % face2_pass_step(op->h.D) != 0))
         return fail(TDG_E_INVALID, "points per pass: FP64 only, a multiple of 8 (3D) or 4 (2D)");
-    op->tile[precision == TDG_FP64 ? 0 : 1] = points_per_pass;
+    const int pi = precision == TDG_FP64 ? 0 : 1;
+    op->tile[pi] = points_per_pass;
+    op->call_family[pi] = -1;
     return 0;
 }
 
@@ -1682,16 +1717,13 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     // best candidate of [0] the tile kernels (family 0), [1] the SIMT kernel, [2] the others
-    // as {time a caller sees, device time}: a call with one launch is issued every 10.2 us from
-    // Python, with two every 12.0, and anything shorter than that hides behind it
-    using Cost = std::pair<double, double>;
-    Cost best[3] = {{1e300, 1e300}, {1e300, 1e300}, {1e300, 1e300}};
+    double best[3] = {1e300, 1e300, 1e300};
     int which[3] = {-1, -1, -1}, n = 0, rc = 0;
     for (size_t i = 0; i < cands.size() && rc == 0; ++i) {
         op->family[pi] = cands[i].family;
         op->ctas[pi] = cands[i].ctas;
         op->tile[pi] = cands[i].tile;
-        for (int w = 0; w < 2 && rc == 0; ++w) rc = tdg_apply(op, precision, x, y, nrhs, ld, stream);
+        for (int w = 0; w < 2 && rc == 0; ++w) rc = apply_as(op, precision, x, y, nrhs, ld, s);
         if (rc == TDG_E_INVALID && cands[i].tile != 0) {  // a points-per-pass that does not fit: skip it
             rc = 0;
             continue;
@@ -1699,7 +1731,7 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
         if (rc) break;
         constexpr int reps = 5;
         cudaEventRecord(e0, s);
-        for (int r = 0; r < reps && rc == 0; ++r) rc = tdg_apply(op, precision, x, y, nrhs, ld, stream);
+        for (int r = 0; r < reps && rc == 0; ++r) rc = apply_as(op, precision, x, y, nrhs, ld, s);
         cudaEventRecord(e1, s);
         cudaEventSynchronize(e1);
         float ms = 0.0f;
@@ -1708,9 +1740,8 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
         if (entries && n < max_entries) entries[n] = tdg_tune_entry{cands[i].family, cands[i].ctas, cands[i].tile, per};
         ++n;
         const int k = std::min(cands[i].family, 2);
-        const Cost cost{std::max(per, k == 2 ? 0.012 : 0.0102), per};
-        if (cost < best[k]) {
-            best[k] = cost;
+        if (per < best[k]) {
+            best[k] = per;
             which[k] = static_cast<int>(i);
         }
     }
@@ -1721,7 +1752,7 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
     // against 18.4 us at 2D p2 Poisson, 18,432 triangles) it therefore stays, though the face-centric
     // kernels would take 12.5 us there.  At 2D p3 Poisson the margin is wider: it is close to both.
     const bool small = h.D == 2 ? h.bs <= 12 : h.N == 1;
-    const bool simt = precision == TDG_FP32 && small && best[1].second < (h.N <= 2 ? 0.95 : 0.8) * best[0].second;
+    const bool simt = precision == TDG_FP32 && small && best[1] < (h.N <= 2 ? 0.95 : 0.8) * best[0];
     int k = best[1] < best[0] ? 1 : 0;
     if (!simt && best[2] < best[k]) k = 2;
     const int bi = which[k];
@@ -1738,6 +1769,7 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
     op->family[pi] = cands[bi].family;
     op->ctas[pi] = cands[bi].ctas;
     op->tile[pi] = cands[bi].tile;
+    op->call_family[pi] = -1;
     if (n_entries) *n_entries = n;
     return 0;
 }
@@ -2259,7 +2291,7 @@ int fgmres(tdg_op* op, int prec, SegPlan const& sp, const double* b, double* x, 
             double* vj = gw.V + static_cast<size_t>(j) * vec;
             double* zj = gw.Z + static_cast<size_t>(j) * vec;
             TDG_TRY(precondition<double>(op, prec, vj, zj, sp.op_nrhs, sp.op_ld, s));
-            TDG_TRY(tdg_apply(op, prec, zj, gw.w, sp.op_nrhs, sp.op_ld, s));
+            TDG_TRY(apply_as(op, prec, zj, gw.w, sp.op_nrhs, sp.op_ld, s));
             const int nv = j + 1;
             const int ng = ngroups(nv);
             // pass 1: h1 = V^T w, w -= V h1
@@ -3043,7 +3075,7 @@ extern "C" int tdg_wave_rhs(tdg_op* op, const double* x, const double* b, double
     auto const& h = op->h;
     if (h.kind != 1) return fail(TDG_E_INVALID, "the wave operator is defined for elasticity");
     if (x == y || (b && b == y)) return fail(TDG_E_INVALID, "y must not alias x or b");
-    TDG_TRY(tdg_apply(op, TDG_FP64, x, y, nrhs, ld, stream));
+    TDG_TRY(apply_as(op, TDG_FP64, x, y, nrhs, ld, static_cast<cudaStream_t>(stream)));
     TDG_TRY(ensure_wave(op));
     int rc = launch_inverse_mass(h.D, h.N, op->wave, h.E, h.Nq, y, b, y, nrhs, ld, static_cast<cudaStream_t>(stream));
     return rc ? fail(rc, "inverse mass launch failed") : 0;
