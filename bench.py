@@ -104,11 +104,16 @@ KERNEL_NAMES = {"tensor": "apply_mma_kernel<Shape<3,4,Elasticity>> (FP64 mma.syn
                 "simt": "apply_kernel<Shape<3,4,Elasticity>, double> (SIMT)"}
 
 
-def launches_per_apply(tune):
-    """Kernel launches of one apply in the fastest configuration of an autotune list: the
-    face-centric families launch a volume and a facet kernel, the others one kernel."""
-    best = min(tune, key=lambda e: e["ms"] if e.get("ms") is not None else 0.0)
-    return 2 if best["family"] in ("face", "face2", "tc05") else 1
+def launches_per_apply(config):
+    """Kernel launches of one apply in a configuration: the face-centric families launch a volume and a
+    facet kernel, the others one kernel."""
+    return 2 if config["family"] in ("face", "face2", "tc05") else 1
+
+
+def kept(op, precision, tune):
+    """The configuration the operator uses, with its measured time from the autotune list."""
+    c = op.apply_config(precision)
+    return dict(c, ms=next((e["ms"] for e in tune if all(e.get(k, 0) == c[k] for k in c)), None))
 
 
 def fp64_peaks(stream) -> dict:
@@ -387,7 +392,7 @@ def run_ours(args):
         tune64 = [{"family": args.family, "ctas_per_sm": args.ctas, "tile": args.tile, "ms": None}]
     else:
         tune64 = op.autotune(FP64, stream=stream)
-    best64 = min(tune64, key=lambda e: e["ms"] or 0.0)
+    best64 = kept(op, FP64, tune64)
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     with ClockSampler(local) as clk:
         for _ in range(args.warmup):
@@ -436,7 +441,7 @@ def run_ours(args):
         tune32 = [{"family": args.family32, "ctas_per_sm": args.ctas, "ms": 0.0}]
     else:
         tune32 = op.autotune(FP32, stream=stream)
-    best32 = min(tune32, key=lambda e: e["ms"])
+    best32 = kept(op, FP32, tune32)
     x32, y32 = x.float(), torch.empty(n, dtype=torch.float32, device="cuda")
     for _ in range(args.warmup):
         op.apply(x32, y32, FP32, stream=stream)
@@ -540,7 +545,7 @@ def run_ours(args):
            "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded mesh, random-field material)",
            "config": cube_config(wl.name, op.E, n, op.Nq, op.nq, world),
            "clocks": clk.summary(), "e2e": e2e,
-           "gpu_launches": args.steps * launches_per_apply([best64]),
+           "gpu_launches": args.steps * launches_per_apply(best64),
            "apply_config": best64, "autotune": tune64,
            "roofline": roofline, "cpu_baseline": cpu,
            "fp32_apply": {"value": world * n / (ms32 * 1e-3), "unit": "DOF/s", "ms_per_step": ms32,
@@ -741,7 +746,7 @@ def run_batch(args):
            "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded meshes, random-field material and force)",
            "config": {"workload": b.name, "problems": args.count, "elements": int(op.E), "dofs": int(n),
                       "sizes": [int(v) for v in b.sizes], "setup_seconds": setup_s},
-           "clocks": clk.summary(), "gpu_launches": args.steps * launches_per_apply(tune["fp64"]), "autotune": tune,
+           "clocks": clk.summary(), "gpu_launches": args.steps * launches_per_apply(op.apply_config(FP64)), "autotune": tune,
            "fp32_apply": {"value": n / (ms32 * 1e-3), "unit": "DOF/s", "ms_per_step": ms32},
            "solve": solve,
            "solve_dof_per_s": {k: n / v["seconds"] for k, v in solve.items() if isinstance(v, dict)}}
@@ -857,7 +862,7 @@ def run_poisson(args):
            "data": "synthetic (tandem GenMesh<2>, sin sin manufactured solution)",
            "config": {"workload": wl.name, "elements": int(op.E), "dofs": int(n),
                       "l2": "L2-resident (14 MB per apply)"},
-           "gpu_launches": args.steps * launches_per_apply(tune["fp64"]), "autotune": tune,
+           "gpu_launches": args.steps * launches_per_apply(op.apply_config(FP64)), "autotune": tune,
            "fp32_apply": {"value": n / (ms32 * 1e-3), "unit": "DOF/s", "ms_per_step": ms32}, "solve": solve}
     print(json.dumps(out), flush=True)
 
@@ -1011,7 +1016,7 @@ def run_vcycle(args):
            "n_gpus": 1, "dtype": "f64", "data": "synthetic (seeded mesh, random-field material)",
            "config": {"workload": wl.name, "dofs": int(op.ndof), "levels": info["degrees"],
                       "smooth_its": MG_SMOOTH_ITS, "coarse_space": "continuous P1"},
-           "coarse_iterations": info["coarse_iterations"] - c0, "apply_config": min(tune, key=lambda e: e["ms"])}
+           "coarse_iterations": info["coarse_iterations"] - c0, "apply_config": kept(op, FP64, tune)}
     print(json.dumps(out), flush=True)
 
 
