@@ -191,9 +191,9 @@ typedef struct {
  * face-centric pair; FP32 also the pair with the tcgen05 volume kernel) at 1 to 4 persistent CTAs
  * per SM (clipped to the occupancy limit of the shape's tile), the FP64 face-centric form also at
  * the tile heights that cover the volume points in 2, 3 and 4 passes, and the SIMT kernel -- with CUDA events on
- * `stream`, and keeps the fastest for later tdg_apply / tdg_solve calls of that precision.  On small
- * shapes (2D up to 12 unknowns per element, 3D degree 1) in FP32 the SIMT kernel, the most accurate,
- * is kept against the face-centric ones where it clearly beats the element-centric one.
+ * `stream`, and keeps the fastest for later tdg_apply / tdg_solve calls of that precision.  In FP32 small
+ * shapes (2D up to 12 unknowns per element, 3D degree 1) keep the SIMT kernel, the most accurate, from a
+ * number of elements x right-hand sides that depends on the shape alone (degree-1 Poisson: always).
  * entries (optional, up to max_entries) receives every measurement; n_entries their count. */
 int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_entry* entries, int max_entries,
                  int* n_entries);

@@ -1678,6 +1678,24 @@ static std::vector<int> face2_tile_candidates(int D, int Nq) {
     return t;
 }
 
+// Elements x right-hand sides from which FP32 applies of this shape keep the SIMT kernel (-1: never).  It sums
+// with FMA in registers and is the most accurate (2-norm against the FP64 apply 7e-8 to 1e-7; face-centric
+// 9e-8 to 1.7e-7, element-centric 1.6e-7 to 2.7e-7), and the small shapes' applies ran it wherever it beat
+// the element-centric kernel.  That line is drawn here by size, so that an operator's rounding does not depend on a
+// measurement: degree-1 Poisson always; else from about the size that fills the GPU once, us SIMT /
+// element-centric just below and above it: 2D p2 Poisson 16.9 / 14.9 and 16.9 / 19.0, p3 19.0 / 21.1 and
+// 23.1 / 30.5, 2D elasticity p1 12.8 / 12.8 and 12.9 / 14.9, p2 21.0 / 16.9 and 23.1 / 28.6, 3D elasticity p1
+// 23.9 / 16.9 and 25.1 / 29.2.  It costs time from there on (face-centric at 2D p3 Poisson, 32,768 triangles:
+// 14.9 us for 41.5); tdg_set_apply_config chooses otherwise.
+static int64_t simt32_from(HostOperator const& h) {
+    const bool poisson = h.kind == 0;
+    if (h.N == 1 && poisson) return 0;
+    if (h.D == 3) return h.N == 1 ? 4500 : -1;
+    if (h.N == 1) return 6000;
+    if (h.N == 2) return poisson ? 12000 : 8400;
+    return h.N == 3 && poisson ? 8400 : -1;
+}
+
 int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_entry* entries, int max_entries,
                  int* n_entries) {
     if (!op || nrhs < 1 || (precision != TDG_FP64 && precision != TDG_FP32))
@@ -1716,9 +1734,8 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    // best candidate of [0] the tile kernels (family 0), [1] the SIMT kernel, [2] the others
-    double best[3] = {1e300, 1e300, 1e300};
-    int which[3] = {-1, -1, -1}, n = 0, rc = 0;
+    double best = 1e300;
+    int bi = -1, n = 0, rc = 0;
     for (size_t i = 0; i < cands.size() && rc == 0; ++i) {
         op->family[pi] = cands[i].family;
         op->ctas[pi] = cands[i].ctas;
@@ -1739,23 +1756,14 @@ int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_ent
         const double per = ms / reps;
         if (entries && n < max_entries) entries[n] = tdg_tune_entry{cands[i].family, cands[i].ctas, cands[i].tile, per};
         ++n;
-        const int k = std::min(cands[i].family, 2);
-        if (per < best[k]) {
-            best[k] = per;
-            which[k] = static_cast<int>(i);
+        if (per < best) {
+            best = per;
+            bi = static_cast<int>(i);
         }
     }
-    // Speed is not the only measure in FP32: the SIMT kernel sums with FMA in registers and is the
-    // most accurate (7e-8 to 1e-7 of the FP64 apply in the 2-norm against 1e-7 to 1.6e-7 of the
-    // face-centric kernels and 1.6e-7 to 2.8e-7 of family 0 below).  On the shapes where it is also
-    // clearly the faster of the two that visit elements (2D up to 12 unknowns, 3D degree 1; 16.9
-    // against 18.4 us at 2D p2 Poisson, 18,432 triangles) it therefore stays, though the face-centric
-    // kernels would take 12.5 us there.  At 2D p3 Poisson the margin is wider: it is close to both.
-    const bool small = h.D == 2 ? h.bs <= 12 : h.N == 1;
-    const bool simt = precision == TDG_FP32 && small && best[1] < (h.N <= 2 ? 0.95 : 0.8) * best[0];
-    int k = best[1] < best[0] ? 1 : 0;
-    if (!simt && best[2] < best[k]) k = 2;
-    const int bi = which[k];
+    const int64_t simt = simt32_from(h);
+    if (precision == TDG_FP32 && simt >= 0 && h.E * nrhs >= simt)
+        bi = static_cast<int>(cands.size()) - 1;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaFree(x);

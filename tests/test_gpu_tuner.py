@@ -52,3 +52,21 @@ def test_call_configuration_serves_single_applies_only():
     assert not torch.equal(y, simt)
     with pytest.raises(_ffi.TdgError, match="bad argument"):
         _ffi.check(_ffi.lib().tdg_set_call_config(op._h, FP64, 4, 0))
+
+
+@pytest.mark.parametrize("kind,dim,n,N,nrhs,simt", [
+    (POISSON, 2, 3, 1, 1, True), (POISSON, 2, 40, 1, 2, True), (POISSON, 3, 2, 1, 1, True),
+    (POISSON, 2, 77, 2, 1, False), (POISSON, 2, 78, 2, 1, True), (POISSON, 2, 9, 2, 75, True),
+    (POISSON, 2, 64, 3, 1, False), (POISSON, 2, 65, 3, 1, True), (ELASTICITY, 2, 54, 1, 1, False),
+    (ELASTICITY, 2, 55, 1, 1, True), (ELASTICITY, 2, 64, 2, 1, False), (ELASTICITY, 2, 65, 2, 1, True),
+    (ELASTICITY, 3, 9, 1, 1, False), (ELASTICITY, 3, 10, 1, 1, True), (ELASTICITY, 2, 40, 3, 4, False)])
+def test_tuner_keeps_the_accurate_fp32_kernel_by_size(kind, dim, n, N, nrhs, simt):
+    op = operator(kind, dim, n, N)
+    for _ in range(3):
+        entries = op.autotune(FP32, nrhs=nrhs)
+        best = min(entries, key=lambda e: e["ms"])
+        kept = op.apply_config(FP32)
+        if simt:
+            assert kept["family"] == "simt"
+        else:
+            assert kept == {k: best[k] for k in ("family", "ctas_per_sm", "tile")}
