@@ -198,7 +198,8 @@ typedef struct {
 int tdg_autotune(tdg_op* op, int precision, int nrhs, void* stream, tdg_tune_entry* entries, int max_entries,
                  int* n_entries);
 /* Sets the apply configuration of `precision` (TDG_FP64 / TDG_FP32; TDG_MIXED and TDG_TF32 follow TDG_FP32)
- * explicitly: kernel family as in tdg_tune_entry and persistent CTAs per SM. */
+ * explicitly: kernel family as in tdg_tune_entry and persistent CTAs per SM.  TDG_MIXED and TDG_TF32 have
+ * no SIMT form and run face-centric under it. */
 int tdg_set_apply_config(tdg_op* op, int precision, int family, int ctas_per_sm);
 /* Another configuration for tdg_apply calls alone, for a caller that needs longer to issue a call than the
  * device needs to run it (one launch may then be quicker than two shorter ones): family -1 takes it back.

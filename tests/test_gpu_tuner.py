@@ -5,7 +5,7 @@ import torch
 
 from cases import make_mesh, material, tandem_quadrature
 from tandem_b200 import _ffi
-from tandem_b200.operator import DGOperator, ELASTICITY, FAMILIES, FP32, FP64, POISSON
+from tandem_b200.operator import DGOperator, ELASTICITY, FAMILIES, FP32, FP64, MIXED, POISSON, TF32
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +70,17 @@ def test_tuner_keeps_the_accurate_fp32_kernel_by_size(kind, dim, n, N, nrhs, sim
             assert kept["family"] == "simt"
         else:
             assert kept == {k: best[k] for k in ("family", "ctas_per_sm", "tile")}
+
+
+@pytest.mark.parametrize("kind,dim,n,N", [(POISSON, 2, 20, 1), (ELASTICITY, 2, 9, 2), (ELASTICITY, 3, 3, 1)])
+@pytest.mark.parametrize("precision", [MIXED, TF32])
+def test_mixed_precisions_run_face_centric_beside_the_simt_kernel(kind, dim, n, N, precision):
+    """The same products as the face-centric configuration, added in FP64 in another order: 1e-12."""
+    op = operator(kind, dim, n, N)
+    x = torch.randn(op.ndof, dtype=torch.float64, device="cuda")
+    y, ref = torch.empty_like(x), torch.empty_like(x)
+    op.set_apply_config(FP32, "face")
+    op.apply(x, ref, precision)
+    op.set_apply_config(FP32, "simt")
+    op.apply(x, y, precision)
+    assert (y - ref).abs().max() <= 1e-12 * ref.abs().max()
