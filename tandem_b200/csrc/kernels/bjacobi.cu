@@ -86,7 +86,7 @@ int run_stream(int64_t E, const TM* inv, const TV* r, TV* z, cudaStream_t s) {
 }
 
 // Inverses up to this size stay in L2 and a row's second access costs nothing: 8,192 blocks of 15
-// (7.9 MB) 3.98 us by rows, 4.27 us streamed; 10,368 blocks of 105 (462 MB) 172 and 120 us.
+// (7.9 MB) 3.98 us by rows, 4.27 us streamed; 10,368 blocks of 105 (462 MB) 172 and 84 us.
 constexpr int64_t kStreamBytes = int64_t(32) << 20;
 
 // Rows, as few groups of up to four columns as they fill, evenly.
