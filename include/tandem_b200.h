@@ -395,6 +395,11 @@ int tdg_mg_info(tdg_op* op, int* nlevels, int max_levels, int* degrees, int* blo
  * (column-major per block, NB = 1 + faces per element) and its neighbour table nbr [E][NB]
  * (slot 0 the element, slot 1 + f the element behind face f, -1 none); for tests. */
 int tdg_mg_level_matrix(tdg_op* op, int level, double* blocks, int32_t* nbr);
+/* y = A x (b NULL) or b - A x of such a level, one device column, as the smoother applies it (FP32 copies of
+ * the blocks under mixed precision): half 0 from whole block rows, else from one block of every symmetric
+ * pair, the form of levels larger than L2 (block sizes 6, 10, 12, 20 and 30); for tests. */
+int tdg_mg_level_apply(tdg_op* op, int level, int half, const double* x, const double* b, double* y,
+                       void* stream);
 /* Host utilities (no device): the level degrees of a strategy (returns their count; degrees may
  * be NULL) and the reference interpolation matrix [Nbf(n_to)][Nbf(n_from)] of one component. */
 int tdg_mg_level_degrees(int strategy, int coarse_degree, int degree, int* degrees);

@@ -61,6 +61,7 @@ SYMBOLS = {
     "tdg_set_preconditioner": (C.c_int, [_p, C.c_int]),
     "tdg_mg_info": (C.c_int, [_p, _p, C.c_int, _p, _p, _p, _p]),
     "tdg_mg_level_matrix": (C.c_int, [_p, C.c_int, _p, _p]),
+    "tdg_mg_level_apply": (C.c_int, [_p, C.c_int, C.c_int, _p, _p, _p, _p]),
     "tdg_mg_level_degrees": (C.c_int, [C.c_int, C.c_int, C.c_int, _p]),
     "tdg_mg_interpolation": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, _p]),
     "tdg_mg_colouring": (C.c_int, [_p, _p, _p]),

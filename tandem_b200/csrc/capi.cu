@@ -2658,6 +2658,30 @@ extern "C" int tdg_mg_level_matrix(tdg_op* op, int level, double* blocks, int32_
     return 0;
 }
 
+extern "C" int tdg_mg_level_apply(tdg_op* op, int level, int half, const double* x, const double* b, double* y,
+                                  void* stream) {
+    if (!op || !x || !y) return fail(TDG_E_INVALID, "null argument");
+    auto const& mg = op->mg;
+    if (!mg.ready) return fail(TDG_E_STATE, "tdg_mg_setup not called");
+    if (level < 0 || level + 1 >= static_cast<int>(mg.lv.size()))
+        return fail(TDG_E_INVALID, "level must be a coarse (block-sparse) level");
+    if (x == y) return fail(TDG_E_INVALID, "x and y must not alias");
+    auto const& L = mg.lv[static_cast<size_t>(level)];
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int64_t E = op->h.E;
+    if (!half) {
+        if (L.A32) return mgk(launch_mg_bsr_apply(E, mg.NB, L.bs, mg.nbr, L.A32, x, b, y, 1, L.n, s), "level apply");
+        return mgk(launch_mg_bsr_apply(E, mg.NB, L.bs, mg.nbr, L.A, x, b, y, 1, L.n, s), "level apply");
+    }
+    DevArena scratch;
+    double* t = nullptr;
+    TDG_CUDA_TRY(scratch.alloc(&t, static_cast<size_t>(E) * mg.NB * L.bs));
+    const int rc = L.A32 ? launch_mg_bsr_half(E, mg.NB, L.bs, mg.nbr, L.A32, x, b, y, t, s)
+                         : launch_mg_bsr_half(E, mg.NB, L.bs, mg.nbr, L.A, x, b, y, t, s);
+    TDG_CUDA_TRY(cudaStreamSynchronize(s));
+    return mgk(rc, "level apply");
+}
+
 extern "C" int tdg_mg_level_degrees(int strategy, int coarse_degree, int degree, int* degrees) {
     try {
         std::vector<int> d = mg_level_degrees(strategy, coarse_degree, degree);

@@ -16,7 +16,7 @@ constexpr int kT = 256;
 
 // Warps per CTA of k_bsr_half: its padded block per group within 48 KB.
 __host__ __device__ constexpr int bsr_half_warps(int bs) {
-    const int epw = bs < 32 ? 32 / bs : 1, per = epw * (bs * (bs | 1) + 2 * bs) * 8;
+    const int epw = 32 / bs, per = epw * (bs * (bs | 1) + 2 * bs) * 8;
     const int w = 48 * 1024 / per;
     return w > 8 ? 8 : (w < 1 ? 1 : w);
 }
@@ -435,20 +435,21 @@ __global__ void __launch_bounds__(kT)
 
 // One right-hand side of a level whose blocks exceed L2: the apply is bound by the blocks' bytes, and
 // the block of element n in row e is the transpose of that of e in row n (the Galerkin operator is
-// symmetric), so each coupling is read once, from its lower element's row: a group of lanes (one per
-// row, BS > 32: two rows each) adds its product to its own result and forms the transposed product
-// from shared memory into t[e][slot], which k_bsr_gather adds to the higher element's row.  Fixed
-// order of summation, no atomics.  Blocks of 30, 10,368 elements: 106 -> 44 us and the gather.
+// symmetric), so each coupling is read once, from its lower element's row: a group of BS lanes (one per
+// row) adds its product to its own result and forms the transposed product from shared memory into
+// t[e][slot], which k_bsr_gather adds to the higher element's row.  Fixed order of summation, no
+// atomics.  Blocks of 30, 10,368 elements: 106 -> 44 us and the gather.
 template <int BS, typename TA>
 __global__ void __launch_bounds__(kT)
     k_bsr_half(int64_t E, int NB, const int32_t* __restrict__ nbr, const TA* __restrict__ A,
                const double* __restrict__ x, double* __restrict__ y, double* __restrict__ t) {
+    static_assert(BS <= 32, "a lane per row");
     let_next_kernel_start();
-    constexpr int GL = BS < 32 ? BS : 32, EPW = 32 / GL, RPL = (BS + 31) / 32, LD = BS | 1;
+    constexpr int EPW = 32 / BS, LD = BS | 1;
     constexpr int WPB = bsr_half_warps(BS);
     __shared__ double s_blk[WPB][EPW][BS * LD];
     __shared__ double s_x[WPB][EPW][2][BS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / GL, l = lane % GL;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / BS, row = lane % BS;
     const bool lane_on = grp < EPW;
     double* sb = s_blk[warp][lane_on ? grp : 0];
     double* xe = s_x[warp][lane_on ? grp : 0][0];
@@ -457,55 +458,39 @@ __global__ void __launch_bounds__(kT)
     for (int64_t w = static_cast<int64_t>(blockIdx.x) * WPB + warp; w < groups; w += static_cast<int64_t>(gridDim.x) * WPB) {
         const int64_t e = w * EPW + grp;
         const bool on = lane_on && e < E;
-        double acc[RPL];
-#pragma unroll
-        for (int i = 0; i < RPL; ++i) acc[i] = 0.0;
+        double acc = 0.0;
         for (int s = 0; s < NB; ++s) {
             const int32_t n = on ? nbr[e * NB + s] : -1;
             const bool use = n >= 0 && (s == 0 || n > e);
             if (!__any_sync(0xffffffffu, use)) continue;
-            double v[RPL][BS];
-#pragma unroll
-            for (int i = 0; i < RPL; ++i) {
-                const int row = l + 32 * i;
+            double v[BS];
+            if (use) {
                 const TA* blk = A + (e * NB + s) * (BS * BS) + row;
-                if (use && row < BS) {
 #pragma unroll
-                    for (int col = 0; col < BS; ++col) v[i][col] = static_cast<double>(blk[col * BS]);
-                    (s == 0 ? xe : xn)[row] = x[static_cast<int64_t>(n) * BS + row];
-                }
+                for (int col = 0; col < BS; ++col) v[col] = static_cast<double>(blk[col * BS]);
+                (s == 0 ? xe : xn)[row] = x[static_cast<int64_t>(n) * BS + row];
             }
             __syncwarp();
             const double* xs = s == 0 ? xe : xn;
+            if (use) {
 #pragma unroll
-            for (int i = 0; i < RPL; ++i) {
-                const int row = l + 32 * i;
-                if (use && row < BS) {
+                for (int col = 0; col < BS; ++col) acc += v[col] * xs[col];
+                if (s > 0)
 #pragma unroll
-                    for (int col = 0; col < BS; ++col) acc[i] += v[i][col] * xs[col];
-                    if (s > 0)
-#pragma unroll
-                        for (int col = 0; col < BS; ++col) sb[col * LD + row] = v[i][col];
-                }
+                    for (int col = 0; col < BS; ++col) sb[col * LD + row] = v[col];
             }
             __syncwarp();
             if (s > 0) {
-#pragma unroll
-                for (int i = 0; i < RPL; ++i) {
-                    const int col = l + 32 * i;
-                    if (use && col < BS) {
-                        double q = 0.0;
+                if (use) {
+                    double q = 0.0;
 #pragma unroll 10
-                        for (int row = 0; row < BS; ++row) q += sb[col * LD + row] * xe[row];
-                        t[(e * NB + s) * BS + col] = q;
-                    }
+                    for (int r = 0; r < BS; ++r) q += sb[row * LD + r] * xe[r];
+                    t[(e * NB + s) * BS + row] = q;
                 }
                 __syncwarp();
             }
         }
-#pragma unroll
-        for (int i = 0; i < RPL; ++i)
-            if (on && l + 32 * i < BS) y[e * BS + l + 32 * i] = acc[i];
+        if (on) y[e * BS + row] = acc;
     }
 }
 
@@ -608,7 +593,7 @@ int launch_mg_bsr_half(int64_t E, int NB, int bs, const int32_t* nbr, const TA* 
     switch (bs) {
 #define TDG_BSR_HALF_CASE(B)                                                                                    \
     case B: {                                                                                                   \
-        constexpr int wpb = bsr_half_warps(B), epw = B < 32 ? 32 / B : 1;                                       \
+        constexpr int wpb = bsr_half_warps(B), epw = 32 / B;                                                   \
         const int64_t need = (E + epw * wpb - 1) / (epw * wpb);                                                 \
         const unsigned g = static_cast<unsigned>(std::min<int64_t>(need, 148 * 16));                            \
         k_bsr_half<B, TA><<<g, 32 * wpb, 0, s>>>(E, NB, nbr, A, x, y, t);                                       \

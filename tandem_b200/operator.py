@@ -395,6 +395,14 @@ class DGOperator:
         _ffi.check(_ffi.lib().tdg_mg_level_matrix(self._h, level, blocks.ctypes.data, nbr.ctypes.data))
         return np.ascontiguousarray(blocks.transpose(0, 1, 3, 2)), nbr
 
+    def mg_level_apply(self, level: int, x, y, b=None, half: bool = False, stream=None) -> None:
+        """y = A x, or b - A x, of a coarse level (tdg_mg_level_apply; for tests)."""
+        n = self.E * self.mg_info()["block_sizes"][level]
+        for v in (x, y) if b is None else (x, y, b):
+            _check_vec(v, FP64, n)
+        _ffi.check(_ffi.lib().tdg_mg_level_apply(self._h, level, int(half), x.data_ptr(),
+                                                 None if b is None else b.data_ptr(), y.data_ptr(), _stream(stream)))
+
     def rhs(self, force_Q: np.ndarray | None = None, bc_q: np.ndarray | None = None) -> np.ndarray:
         """Right-hand side (DGOperator::rhs): force_Q [E, Q, Nq], bc_q [F, Q, nq]."""
         b = np.zeros(self.ndof)
