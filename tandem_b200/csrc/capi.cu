@@ -446,13 +446,14 @@ int upload_warp(tdg_op* op, DevArena& arena) {
     std::vector<int> fids;
     facet_tiles(h, 8, fids, ftiles);
     const WarpFacetTables ft = warp_facet_tables(h);
+    const FaceFrames frames(h);
     const int64_t nft = static_cast<int64_t>(ftiles.size()), fs = warp_facet_stride(h);
     std::vector<double> fct(static_cast<size_t>(nft) * fs, 0.0);
     std::vector<int4> tids(static_cast<size_t>(nft) * 8, make_int4(-1, -1, -1, 0));
 #pragma omp parallel for schedule(static)
     for (int64_t t = 0; t < nft; ++t) {
         const int4 td = ftiles[t];
-        warp_facet_tile(h, &fids[td.x], td.y, &fct[static_cast<size_t>(t) * fs]);
+        warp_facet_tile(h, frames, &fids[td.x], td.y, &fct[static_cast<size_t>(t) * fs]);
         for (int te = 0; te < td.y; ++te) {
             const int f = fids[td.x + te];
             tids[static_cast<size_t>(t) * 8 + te] =
@@ -491,6 +492,7 @@ int upload_warp32(tdg_op* op, DevArena& arena) {
     std::vector<int> fids;
     facet_tiles(h, 16, fids, ftiles);
     const WarpFacetTables32 ft = warp_facet_tables32(h);
+    const FaceFrames frames(h);
     const int64_t nft = static_cast<int64_t>(ftiles.size()), fs = warp_facet_stride32(h);
     std::vector<float> fct(static_cast<size_t>(nft) * fs, 0.0f);
     std::vector<double> pen(static_cast<size_t>(nft) * 16, 0.0);
@@ -498,7 +500,7 @@ int upload_warp32(tdg_op* op, DevArena& arena) {
 #pragma omp parallel for schedule(static)
     for (int64_t t = 0; t < nft; ++t) {
         const int4 td = ftiles[t];
-        warp_facet_tile32(h, &fids[td.x], td.y, &fct[static_cast<size_t>(t) * fs]);
+        warp_facet_tile32(h, frames, &fids[td.x], td.y, &fct[static_cast<size_t>(t) * fs]);
         for (int te = 0; te < td.y; ++te) {
             const int f = fids[td.x + te];
             pen[static_cast<size_t>(t) * 16 + te] = h.penalty[f];

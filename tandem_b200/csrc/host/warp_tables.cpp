@@ -270,7 +270,7 @@ namespace {
 // J^-1 in the face-adapted directions (Ti) / w n and the last shared one; Poisson w n . (K G) (the flux
 // and the lift both contract with it) / the last one: `scale` x w |n|.
 template <class Put>
-void facet_point_fields(HostOperator const& h, int64_t f, int q, double const (*Ti)[9], double scale, Put&& put) {
+void facet_point_fields(HostOperator const& h, int64_t f, int q, double const* const (&Ti)[2], double scale, Put&& put) {
     const int D = h.D, DD = D * D, nq = h.nq;
     const double wq = h.w[q], last = scale * (wq * h.fNl[static_cast<size_t>(f) * nq + q]);
     double n[3];
@@ -335,11 +335,16 @@ Slot slot32(Blocks const& b, int fields, int te, int q) {
 
 }  // namespace
 
-void warp_facet_tile(HostOperator const& h, int const* fids, int count, double* out) {
+FaceFrames::FaceFrames(HostOperator const& h) {
+    double T[9];
+    for (int f = 0; f < h.nfaces; ++f) face_directions(h.D, f, T, inv[f]);
+}
+
+void warp_facet_tile(HostOperator const& h, FaceFrames const& frames, int const* fids, int count, double* out) {
     const int nf = facet_fields(h);
     const Blocks blk(h.nq);
-    double T[9], Ti[2][9];
-    for (int s = 0; s < 2; ++s) face_directions(h.D, h.loc[2 * static_cast<int64_t>(fids[0]) + s], T, Ti[s]);
+    int32_t const* l = &h.loc[2 * static_cast<int64_t>(fids[0])];
+    double const* const Ti[2] = {frames.inv[l[0]], frames.inv[l[1]]};
     for (int te = 0; te < count; ++te)
         for (int q = 0; q < h.nq; ++q) {
             const Slot sl = facet_slot(h, blk, nf, te, q);
@@ -434,11 +439,11 @@ int64_t warp_volume_stride32(HostOperator const& h) {
     return static_cast<int64_t>(volume_fields(h)) * (128 * blk.full + 64 * blk.half);
 }
 
-void warp_facet_tile32(HostOperator const& h, int const* fids, int count, float* out) {
+void warp_facet_tile32(HostOperator const& h, FaceFrames const& frames, int const* fids, int count, float* out) {
     const int nf = facet_fields(h);
     const Blocks blk(h.nq);
-    double T[9], Ti[2][9];
-    for (int s = 0; s < 2; ++s) face_directions(h.D, h.loc[2 * static_cast<int64_t>(fids[0]) + s], T, Ti[s]);
+    int32_t const* l = &h.loc[2 * static_cast<int64_t>(fids[0])];
+    double const* const Ti[2] = {frames.inv[l[0]], frames.inv[l[1]]};
     for (int te = 0; te < count; ++te)
         for (int q = 0; q < h.nq; ++q) {
             const Slot sl = slot32(blk, nf, te, q);

@@ -23,10 +23,16 @@ std::vector<double> warp_volume_frags(HostOperator const& h);
 int64_t warp_volume_stride(HostOperator const& h);
 void warp_volume_tile(HostOperator const& h, int64_t tile, double* out);
 
+// Inverses of the faces' adapted reference directions, formed once: the tiles are filled in parallel and
+// allocate nothing there (an exception cannot leave a parallel region).
+struct FaceFrames {
+    double inv[4][9];
+    explicit FaceFrames(HostOperator const& h);
+};
 // Facet geometry of one tile of up to 8 facets of one (l0, l1): `count` facet ids at `fids`; out
 // holds warp_facet_stride(h) doubles, zeroed.
 int64_t warp_facet_stride(HostOperator const& h);
-void warp_facet_tile(HostOperator const& h, int const* fids, int count, double* out);
+void warp_facet_tile(HostOperator const& h, FaceFrames const& frames, int const* fids, int count, double* out);
 
 // The same for the FP32 kernels (kernels/apply_warp32.cuh): tiles of 16, fragments [table][fragment]
 // [lane][2]; the facet geometry's last shared field lacks the penalty.
@@ -39,7 +45,7 @@ WarpFacetTables32 warp_facet_tables32(HostOperator const& h);
 std::vector<float> warp_volume_frags32(HostOperator const& h);
 int64_t warp_facet_stride32(HostOperator const& h);
 int64_t warp_volume_stride32(HostOperator const& h);
-void warp_facet_tile32(HostOperator const& h, int const* fids, int count, float* out);
+void warp_facet_tile32(HostOperator const& h, FaceFrames const& frames, int const* fids, int count, float* out);
 void warp_volume_tile32(HostOperator const& h, int64_t tile, float* out);
 
 }  // namespace tdg
