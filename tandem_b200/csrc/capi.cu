@@ -22,6 +22,7 @@
 #include <cstring>
 #include <exception>
 #include <limits>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <utility>
@@ -157,13 +158,17 @@ struct DevArena {
         return e;
     }
     template <typename T>
-    cudaError_t upload(T const** out, std::vector<T> const& h) {
+    cudaError_t upload(T const** out, T const* h, size_t n) {
         T* d = nullptr;
-        cudaError_t e = alloc(&d, h.size());
+        cudaError_t e = alloc(&d, n);
         if (e != cudaSuccess) return e;
-        e = cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+        e = cudaMemcpy(d, h, n * sizeof(T), cudaMemcpyHostToDevice);
         *out = d;
         return e;
+    }
+    template <typename T>
+    cudaError_t upload(T const** out, std::vector<T> const& h) {
+        return upload(out, h.data(), h.size());
     }
     void release() {
         for (void* p : ptrs) cudaFree(p);
@@ -448,7 +453,9 @@ int upload_warp(tdg_op* op, DevArena& arena) {
     const WarpFacetTables ft = warp_facet_tables(h);
     const FaceFrames frames(h);
     const int64_t nft = static_cast<int64_t>(ftiles.size()), fs = warp_facet_stride(h);
-    std::vector<double> fct(static_cast<size_t>(nft) * fs, 0.0);
+    // uninitialised: the thread that fills a tile touches (and zeroes) its memory first
+    const size_t nfct = static_cast<size_t>(nft) * fs;
+    std::unique_ptr<double[]> fct(new double[nfct]);
     std::vector<int4> tids(static_cast<size_t>(nft) * 8, make_int4(-1, -1, -1, 0));
 #pragma omp parallel for schedule(static)
     for (int64_t t = 0; t < nft; ++t) {
@@ -461,11 +468,12 @@ int upload_warp(tdg_op* op, DevArena& arena) {
         }
     }
     const int64_t nvt = (h.E + 7) / 8, vs = warp_volume_stride(h);
-    std::vector<double> vol(static_cast<size_t>(nvt) * vs, 0.0);
+    const size_t nvol = static_cast<size_t>(nvt) * vs;
+    std::unique_ptr<double[]> vol(new double[nvol]);
 #pragma omp parallel for schedule(static)
     for (int64_t t = 0; t < nvt; ++t) warp_volume_tile(h, t, &vol[static_cast<size_t>(t) * vs]);
     if (nft) {
-        TDG_CUDA_TRY(arena.upload(&wg.fct, fct));
+        TDG_CUDA_TRY(arena.upload(&wg.fct, fct.get(), nfct));
         TDG_CUDA_TRY(arena.upload(&wg.ftiles, ftiles));
         TDG_CUDA_TRY(arena.upload(&wg.tids, tids));
     }
@@ -473,7 +481,7 @@ int upload_warp(tdg_op* op, DevArena& arena) {
     TDG_CUDA_TRY(arena.upload(&wg.ftab, ft.frags));
     TDG_CUDA_TRY(arena.upload(&wg.fperm, ft.perm));
     TDG_CUDA_TRY(arena.upload(&wg.vtab, warp_volume_frags(h)));
-    TDG_CUDA_TRY(arena.upload(&wg.vol, vol));
+    TDG_CUDA_TRY(arena.upload(&wg.vol, vol.get(), nvol));
     {
         const int* st = nullptr;
         TDG_CUDA_TRY(arena.upload(&st, std::vector<int>(1, 0)));
@@ -494,7 +502,8 @@ int upload_warp32(tdg_op* op, DevArena& arena) {
     const WarpFacetTables32 ft = warp_facet_tables32(h);
     const FaceFrames frames(h);
     const int64_t nft = static_cast<int64_t>(ftiles.size()), fs = warp_facet_stride32(h);
-    std::vector<float> fct(static_cast<size_t>(nft) * fs, 0.0f);
+    const size_t nfct = static_cast<size_t>(nft) * fs;
+    std::unique_ptr<float[]> fct(new float[nfct]);
     std::vector<double> pen(static_cast<size_t>(nft) * 16, 0.0);
     std::vector<int4> tids(static_cast<size_t>(nft) * 16, make_int4(-1, -1, -1, 0));
 #pragma omp parallel for schedule(static)
@@ -509,11 +518,12 @@ int upload_warp32(tdg_op* op, DevArena& arena) {
         }
     }
     const int64_t nvt = (h.E + 15) / 16, vs = warp_volume_stride32(h);
-    std::vector<float> vol(static_cast<size_t>(nvt) * vs, 0.0f);
+    const size_t nvol = static_cast<size_t>(nvt) * vs;
+    std::unique_ptr<float[]> vol(new float[nvol]);
 #pragma omp parallel for schedule(static)
     for (int64_t t = 0; t < nvt; ++t) warp_volume_tile32(h, t, &vol[static_cast<size_t>(t) * vs]);
     if (nft) {
-        TDG_CUDA_TRY(arena.upload(&wg.fct, fct));
+        TDG_CUDA_TRY(arena.upload(&wg.fct, fct.get(), nfct));
         TDG_CUDA_TRY(arena.upload(&wg.pen, pen));
         TDG_CUDA_TRY(arena.upload(&wg.ftiles, ftiles));
         TDG_CUDA_TRY(arena.upload(&wg.tids, tids));
@@ -522,7 +532,7 @@ int upload_warp32(tdg_op* op, DevArena& arena) {
     TDG_CUDA_TRY(arena.upload(&wg.ftab, ft.frags));
     TDG_CUDA_TRY(arena.upload(&wg.fperm, ft.perm));
     TDG_CUDA_TRY(arena.upload(&wg.vtab, warp_volume_frags32(h)));
-    TDG_CUDA_TRY(arena.upload(&wg.vol, vol));
+    TDG_CUDA_TRY(arena.upload(&wg.vol, vol.get(), nvol));
     wg.status = op->tc32.status;
     wg.nftiles = static_cast<int>(nft);
     op->warp32 = wg;

@@ -341,6 +341,7 @@ FaceFrames::FaceFrames(HostOperator const& h) {
 }
 
 void warp_facet_tile(HostOperator const& h, FaceFrames const& frames, int const* fids, int count, double* out) {
+    std::fill_n(out, warp_facet_stride(h), 0.0);
     const int nf = facet_fields(h);
     const Blocks blk(h.nq);
     int32_t const* l = &h.loc[2 * static_cast<int64_t>(fids[0])];
@@ -354,6 +355,7 @@ void warp_facet_tile(HostOperator const& h, FaceFrames const& frames, int const*
 }
 
 void warp_volume_tile(HostOperator const& h, int64_t tile, double* out) {
+    std::fill_n(out, warp_volume_stride(h), 0.0);
     const int nf = volume_fields(h);
     const Blocks blk(h.Nq);
     for (int te = 0; te < 8 && tile * 8 + te < h.E; ++te)
@@ -440,6 +442,7 @@ int64_t warp_volume_stride32(HostOperator const& h) {
 }
 
 void warp_facet_tile32(HostOperator const& h, FaceFrames const& frames, int const* fids, int count, float* out) {
+    std::fill_n(out, warp_facet_stride32(h), 0.0f);
     const int nf = facet_fields(h);
     const Blocks blk(h.nq);
     int32_t const* l = &h.loc[2 * static_cast<int64_t>(fids[0])];
@@ -453,6 +456,7 @@ void warp_facet_tile32(HostOperator const& h, FaceFrames const& frames, int cons
 }
 
 void warp_volume_tile32(HostOperator const& h, int64_t tile, float* out) {
+    std::fill_n(out, warp_volume_stride32(h), 0.0f);
     const int nf = volume_fields(h);
     const Blocks blk(h.Nq);
     for (int te = 0; te < 16 && tile * 16 + te < h.E; ++te)

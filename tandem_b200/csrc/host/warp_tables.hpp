@@ -19,7 +19,8 @@ WarpFacetTables warp_facet_tables(HostOperator const& h);
 
 // Volume fragments.
 std::vector<double> warp_volume_frags(HostOperator const& h);
-// Volume geometry of the tile of elements [8 tile, 8 tile + 8): warp_volume_stride(h) doubles, zeroed.
+// Volume geometry of the tile of elements [8 tile, 8 tile + 8): warp_volume_stride(h) doubles (zero
+// where there is no element or point).
 int64_t warp_volume_stride(HostOperator const& h);
 void warp_volume_tile(HostOperator const& h, int64_t tile, double* out);
 
@@ -30,7 +31,7 @@ struct FaceFrames {
     explicit FaceFrames(HostOperator const& h);
 };
 // Facet geometry of one tile of up to 8 facets of one (l0, l1): `count` facet ids at `fids`; out
-// holds warp_facet_stride(h) doubles, zeroed.
+// holds warp_facet_stride(h) doubles.
 int64_t warp_facet_stride(HostOperator const& h);
 void warp_facet_tile(HostOperator const& h, FaceFrames const& frames, int const* fids, int count, double* out);
 
