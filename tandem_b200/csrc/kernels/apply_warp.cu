@@ -12,7 +12,7 @@ namespace {
 template <class S, bool TG>
 int launch_facets(int nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld, cudaStream_t s,
                   int ctas, bool early, int most, size_t tab, size_t per_warp) {
-    static bool ready = false;
+    static PerDevice ready;
     auto kern = facew_kernel<S, TG>;
     if (int rc = allow_shared(kern, ready)) return rc;
     const int64_t nwork = static_cast<int64_t>(wg.nftiles) * nrhs;
@@ -40,7 +40,7 @@ int run_facets(int nq, WarpGeo const& wg, const double* x, double* y, int nrhs, 
 template <class S, bool TG>
 int launch_volume(int64_t E, int Nq, WarpGeo const& wg, const double* x, double* y, int nrhs, int64_t ld,
                   cudaStream_t s, int ctas, int most, size_t tab, size_t per_warp) {
-    static bool ready = false;
+    static PerDevice ready;
     auto kern = volw_kernel<S, TG>;
     if (int rc = allow_shared(kern, ready)) return rc;
     const int64_t nwork = (E + 7) / 8 * nrhs;

@@ -12,7 +12,7 @@ namespace {
 template <class S, typename TX, int NP, bool TG>
 int go_facets(int nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs, int64_t ld, cudaStream_t s, int ctas, bool early,
               int most, size_t tab, size_t per_warp) {
-    static bool ready = false;
+    static PerDevice ready;
     auto kern = facew32_kernel<S, TX, NP, TG>;
     if (int rc = allow_shared(kern, ready)) return rc;
     const int64_t nwork = static_cast<int64_t>(wg.nftiles) * nrhs;
@@ -40,7 +40,7 @@ int run_facets32(int nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs, int6
 template <class S, typename TX, int NP, bool TG>
 int go_volume(int64_t E, int Nq, WarpGeo32 const& wg, const TX* x, TX* y, int nrhs, int64_t ld, cudaStream_t s,
               int ctas, int most, size_t tab, size_t per_warp) {
-    static bool ready = false;
+    static PerDevice ready;
     auto kern = volw32_kernel<S, TX, NP, TG>;
     if (int rc = allow_shared(kern, ready)) return rc;
     const int64_t nwork = (E + 15) / 16 * nrhs;

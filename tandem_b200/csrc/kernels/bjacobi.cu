@@ -1,6 +1,7 @@
 // Instances and launchers of the block-Jacobi kernels.
 #include "bjacobi.cuh"
 #include "dispatch.hpp"
+#include "per_device.hpp"
 
 #include "../../../include/tandem_b200.h"
 
@@ -69,15 +70,16 @@ int run_stream(int64_t E, const TM* inv, const TV* r, TV* z, cudaStream_t s) {
     using L = BjacStream<BS, TM>;
     constexpr size_t smem = L::smem(sizeof(TV));
     auto kern = bjac_stream_kernel<BS, TM, TV>;
-    static int per_sm = 0;
-    if (per_sm == 0) {
+    static PerDevice resident;
+    const int per_sm = resident.get([&] {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
             cudaSuccess)
-            return TDG_E_CUDA;
+            return 0;
         int n = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 256, smem) != cudaSuccess || n < 1) n = 1;
-        per_sm = n;
-    }
+        return n;
+    });
+    if (per_sm < 1) return TDG_E_CUDA;
     const int64_t pairs = ((E + L::TE - 1) / L::TE + 1) / 2;  // two teams per CTA
     int64_t grid = static_cast<int64_t>(device_sm_count()) * per_sm;
     if (grid > pairs) grid = pairs;

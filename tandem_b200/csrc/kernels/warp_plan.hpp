@@ -4,6 +4,7 @@
 #include "apply_warp.cuh"
 #include "dispatch.hpp"
 #include "early.cuh"
+#include "per_device.hpp"
 
 #include "../../../include/tandem_b200.h"
 
@@ -14,13 +15,14 @@ namespace tdg {
 
 // Dynamic shared memory a CTA may take beside the kernels' static arrays.
 inline size_t shared_limit() {
-    static const size_t limit = [] {
+    static PerDevice limit;
+    const int v = limit.get([] {
         int dev = 0, optin = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        return optin > 2048 ? static_cast<size_t>(optin) - 2048 : size_t(0);
-    }();
-    return limit;
+        return optin - 2048;
+    });
+    return v > 0 ? static_cast<size_t>(v) : size_t(0);
 }
 
 // Grid, warps per CTA (one persistent CTA per SM) and split of `nwork` items of `nblk` blocks each.
@@ -67,13 +69,12 @@ int launch_facet_kernel(bool early, void (*kern)(P...), int grid, int threads, s
 }
 
 template <class K>
-int allow_shared(K kern, bool& ready) {
-    if (ready) return 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared_limit())) !=
-        cudaSuccess)
-        return TDG_E_CUDA;
-    ready = true;
-    return 0;
+int allow_shared(K kern, PerDevice& ready) {
+    const int ok = ready.get([&] {
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared_limit())) ==
+               cudaSuccess;
+    });
+    return ok > 0 ? 0 : TDG_E_CUDA;
 }
 
 }  // namespace tdg
