@@ -1497,6 +1497,21 @@ int tdg_facet_normals(const tdg_op* op, double* out) {
     return 0;
 }
 
+// The operator's device data (both precisions, the penalty) goes; the next call uploads it again.  The
+// pointers go with it: a solve reads the status words of both precisions.
+static void release_operator_data(tdg_op* op) {
+    op->arena64.release();
+    op->arena32.release();
+    op->arena_common.release();
+    op->uploaded64 = op->uploaded32 = false;
+    op->penalty = nullptr;
+    op->sides = nullptr;
+    op->mma = MmaTiles{};
+    op->tc32 = Tc32Tiles{};
+    op->warp = WarpGeo{};
+    op->warp32 = WarpGeo32{};
+}
+
 int tdg_set_material(tdg_op* op, const double* c0_Q, const double* c1_Q) {
     if (!op) return fail(TDG_E_INVALID, "null operator");
     try {
@@ -1504,13 +1519,8 @@ int tdg_set_material(tdg_op* op, const double* c0_Q, const double* c1_Q) {
     } catch (std::exception const& e) {
         return fail(TDG_E_INVALID, e.what());
     }
-    op->arena64.release();
-    op->arena32.release();
-    op->arena_common.release();
+    release_operator_data(op);
     op->arena_pc.release();
-    op->uploaded64 = op->uploaded32 = false;
-    op->penalty = nullptr;
-    op->sides = nullptr;
     op->blk = nullptr;
     op->inv = nullptr;
     op->inv_precision = -1;
@@ -1531,12 +1541,7 @@ int tdg_update_material(tdg_op* op, const double* c0_Q, const double* c1_Q) {
     }
     // the operator's own data (both precisions, the penalty) follow the new material on the next
     // upload; the block-Jacobi inverses (arena_pc) and the multigrid hierarchy stay as they are
-    op->arena64.release();
-    op->arena32.release();
-    op->arena_common.release();
-    op->uploaded64 = op->uploaded32 = false;
-    op->penalty = nullptr;
-    op->sides = nullptr;
+    release_operator_data(op);
     return 0;
 }
 
