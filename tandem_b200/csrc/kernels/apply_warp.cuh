@@ -133,7 +133,10 @@ __device__ __forceinline__ bool load_tables(double* dst, const double* src, int 
     }
     __syncthreads();
     const bool ok = mbar_wait_bounded(bar, 0);
-    if (!ok && threadIdx.x == 0 && status) atomicExch(status, 1);
+    if (!ok) {
+        if (threadIdx.x == 0 && status) atomicExch(status, 1);
+        mbar_wait_bounded(bar, 0);  // once more: the copy must not outlive the CTA
+    }
     return __syncthreads_and(ok) != 0;
 }
 
@@ -473,17 +476,18 @@ __global__ void __launch_bounds__(32 * WarpTile<S>::FWARPS, 1)
     const auto side_geo = [&](Item const& it, int side, int b) {
         return wg.fct + it.tile * gstride + b * (L::FF * 64) + (side ? L::SF * (b < blk.full ? 64 : 32) : 0);
     };
+    bool ok = true;  // this lane's waits have ended in time
     const auto issue = [&](Item const& it, int side, int b) {  // starts their copy into the warp's buffer
-        if (lane == 0)
+        if (lane == 0 && ok)
             bulk_load(gbuf, side_geo(it, side, b),
                       static_cast<unsigned>(facet_side_doubles<S>(b < blk.full ? 2 : 1) * sizeof(double)), &s_gbar[warp]);
     };
     unsigned parity = 0;
-    bool ok = true;
     const auto arrived = [&] {
         if (ok && !mbar_wait_bounded(&s_gbar[warp], parity)) {
-            ok = false;  // no further waits; the host reads the status word
+            ok = false;  // no further waits and copies; the host reads the status word
             if (wg.status) atomicExch(wg.status, 1);
+            mbar_wait_bounded(&s_gbar[warp], parity);  // once more: the copy in flight must not outlive the CTA
         }
         parity ^= 1;
     };
