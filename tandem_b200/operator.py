@@ -207,36 +207,34 @@ class DGOperator:
         """On the smallest operators a call of this class takes longer to issue than the device needs: the
         face-centric pair's two launches then cost more than one longer kernel (2D p1 Poisson, 162
         triangles: 11.8 us per call for 7.8 us on the device, 10.3 with one launch of 10.2).  A call costs the
-        longer of its device time and its issue interval, measured here on both; where one launch costs
-        less, it serves single applies (tdg_set_call_config); solves and captures keep the device's
-        choice.  FP32: the SIMT kernel alone may step in, the only one at least as accurate."""
+        longer of its device time and its issue interval, measured here; where one launch costs less, it
+        serves single applies (tdg_set_call_config); solves and captures keep the device's choice.
+        FP32: the SIMT kernel alone may step in, the only one at least as accurate."""
         import torch
         kept = self.apply_config(precision)
         ms = min((e["ms"] for e in entries if all(e[k] == kept[k] for k in kept)), default=0.0)
         one = min((e for e in entries if e["family"] == "simt" or (e["family"] == "tensor" and precision == FP64)),
                   key=lambda e: e["ms"], default=None)
-        if kept["family"] not in ("face", "face2", "tc05") or one is None or one["ms"] > 0.05:  # no call takes that long to issue
-            return
+        if kept["family"] not in ("face", "face2", "tc05") or one is None or one["ms"] > 0.025:
+            return  # longer than a call takes to issue (12 us): no need to measure that
         x = torch.zeros(nrhs * self.ndof, dtype=torch.float32 if precision == FP32 else torch.float64, device="cuda")
         y = torch.empty_like(x)
 
-        def issue_ms() -> float:
-            best = np.inf
-            for _ in range(3):
-                torch.cuda.synchronize()
-                t = time.perf_counter()
-                for _ in range(8):
-                    self.apply(x, y, precision, nrhs=nrhs, stream=stream)
-                best = min(best, (time.perf_counter() - t) / 8)
+        def call_ms(device_ms: float) -> float:  # or the median interval between calls, past the first few
             torch.cuda.synchronize()
-            return best * 1e3
+            t = []
+            for _ in range(25):
+                self.apply(x, y, precision, nrhs=nrhs, stream=stream)
+                t.append(time.perf_counter())
+            torch.cuda.synchronize()
+            return max(device_ms, float(np.median(np.diff(t[4:]))) * 1e3)
 
-        pair = max(issue_ms(), ms)
+        pair = call_ms(ms)
         if pair <= one["ms"]:
             return
         set_call = _ffi.lib().tdg_set_call_config
         _ffi.check(set_call(self._h, precision, FAMILIES.index(one["family"]), one["ctas_per_sm"]))
-        if max(issue_ms(), one["ms"]) >= pair:
+        if call_ms(one["ms"]) > 0.95 * pair:
             _ffi.check(set_call(self._h, precision, -1, 0))
 
     def set_apply_config(self, precision: int, family: str, ctas_per_sm: int = 0, tile: int = 0) -> None:
