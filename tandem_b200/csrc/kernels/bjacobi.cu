@@ -91,32 +91,35 @@ int run_stream(int64_t E, const TM* inv, const TV* r, TV* z, cudaStream_t s) {
 // (7.9 MB) 3.98 us by rows, 4.27 us streamed; 10,368 blocks of 105 (462 MB) 172 and 84 us.
 constexpr int64_t kStreamBytes = int64_t(32) << 20;
 
-// Rows, as few groups of up to four columns as they fill, evenly.
+// Rows, as few groups of up to five columns as they fill, evenly.
 template <int BS, typename TM, typename TV>
 int run_row_groups(int64_t E, const TM* inv, const TV* r, TV* z, int nrhs, int64_t ld, cudaStream_t s) {
-    const int groups = (nrhs + 3) / 4;
+    const int groups = (nrhs + 4) / 5;
     switch ((nrhs + groups - 1) / groups) {
         case 1: return run_rows<BS, TM, TV, 1>(E, inv, r, z, nrhs, ld, s);
         case 2: return run_rows<BS, TM, TV, 2>(E, inv, r, z, nrhs, ld, s);
         case 3: return run_rows<BS, TM, TV, 3>(E, inv, r, z, nrhs, ld, s);
-        default: return run_rows<BS, TM, TV, 4>(E, inv, r, z, nrhs, ld, s);
+        case 4: return run_rows<BS, TM, TV, 4>(E, inv, r, z, nrhs, ld, s);
+        default: return run_rows<BS, TM, TV, 5>(E, inv, r, z, nrhs, ld, s);
     }
 }
 
 // One right-hand side: bound by the inverses, streamed.  Several: by rows, each column apart, while all of
 // them fit beside each other (a CTA and column per quarter of an SM); else on the tensor pipe (FP64
 // vectors, blocks from 10: below, a fragment is mostly padding), where eight columns cost what one
-// does: from five columns on, or from two where four warps share an element.  105 x 105 blocks in FP32
-// take rows up to four columns too: the conversions of their entries bound the tensor form.  us, by rows / tensor
-// pipe: 35 x 35, 6,000 elements, 2 columns 11.6 / 23.0, 4 19.1 / 23.1, 8 31.4 / 24.0; 105 x 105, 6,000 elements,
-// 2 columns 116 / 94 (FP32 inverses 89 / 152), 8 257 / 112; 30 x 30, 48 elements, 8 columns 4.8 / 6.5.
+// does: from five columns on, or from two where four warps share an element.  The conversions of FP32
+// inverses weigh on the tensor form, so above 16 they take rows up to five columns, the 105 x 105
+// ones too.  us, by rows / tensor pipe: 35 x 35, 6,000 elements, 2 columns 11.6 / 23.0, 4 19.1 / 23.1, 8 31.4 /
+// 24.0, FP32 inverses 5 18.9 / 25.0; 105 x 105, 6,000 elements, 2 columns 116 / 94 (FP32 inverses 89 / 152),
+// 8 257 / 112; 30 x 30, 48 elements, 8 columns 4.8 / 6.5.
 template <int BS, typename TM, typename TV>
 int run_bapply(int64_t E, const TM* inv, const TV* r, TV* z, int nrhs, int64_t ld, cudaStream_t s) {
     if (nrhs == 1 && E * bjac_packed_size(BS) * static_cast<int64_t>(sizeof(TM)) >= kStreamBytes)
         return run_stream<BS, TM, TV>(E, inv, r, z, s);
     if constexpr (std::is_same_v<TV, double> && BS >= 10) {
         constexpr int cols = 8 * bjac_mma_tiles<BS>(), epc = 4 / bjac_mma_warps<BS>();
-        constexpr int few = bjac_mma_warps<BS>() == 1 || (BS > 60 && sizeof(TM) == 4) ? 4 : 1;  // columns taken by rows
+        constexpr bool one = bjac_mma_warps<BS>() == 1, f32 = sizeof(TM) == 4;
+        constexpr int few = f32 && BS > 16 && (one || BS > 60) ? 5 : (one ? 4 : 1);  // columns taken by rows
         constexpr int te = 256 / BS;
         const bool beside = few > 1 && (E + te - 1) / te * nrhs <= 4 * static_cast<int64_t>(device_sm_count());
         if (nrhs > few && !beside) {

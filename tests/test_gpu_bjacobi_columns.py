@@ -1,5 +1,5 @@
 """Block-Jacobi apply to several columns, by each route of its dispatch: every column apart (all rows fit
-beside each other), rows in groups of two to four columns, the FP64 tensor pipe with one warp per element and with
+beside each other), rows in groups of two to five columns, the FP64 tensor pipe with one warp per element and with
 four.  Checked against dense solves with the operator's own diagonal blocks, in place and at a
 padded stride, with partial groups.  And the time: columns together never cost much more than one by one.
 
