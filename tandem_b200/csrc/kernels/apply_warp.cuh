@@ -26,9 +26,9 @@
 // table and differ only in the order of the basis functions (modal bases keep one per face).
 //
 // Measured on a B200 (whole apply, against the CTA-wide tile GEMMs through shared memory that these
-// kernels replaced): 3D p4 elasticity, 48,000 tetrahedra 665 -> 368 us (volume 144, facets 220; the
+// kernels replaced): 3D p4 elasticity, 48,000 tetrahedra 665 -> 365 us (volume 144, facets 220 apart; the
 // products alone take 108 and 113 us of the FP64 pipe, the flux arithmetic 11 and 27); 2D p4 Poisson,
-// 29,000 triangles x 32 columns 593 -> 246 us; 8,192 triangles 18.4 -> 12.8 us.  Facet atomics are
+// 17,712 triangles x 32 columns 593 -> 238 us; 8,192 triangles 18.4 -> 11.8 us.  Facet atomics are
 // not on the critical path (plain stores time the same).
 //
 // Facet modes: 1 interior flux, both sides; 2 boundary (Dirichlet / fault) flux, side 0; 3 interior

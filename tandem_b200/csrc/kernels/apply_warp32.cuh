@@ -5,11 +5,13 @@
 // backward product's A fragment {a0, a2, a1, a3} (k index t = point 2t, t + 4 = point 2t + 1).
 // TX is the vectors' type: float, or double (x rounded to FP32 on load, y accumulated in FP64).
 //
-// Bound by issue: the splits, the flux arithmetic and the products share the schedulers.  Measured on
-// a B200, FP32 vectors, against the tile products of a whole CTA behind the tcgen05 volume kernel that
-// stood here before: 3D p4 elasticity, 24,576 tetrahedra 172 us (volume 64, facets 115, overlapping; before
-// 242: 82 and 160); 3D p2 elasticity, 7,986 tetrahedra 23 us (39); 3D p3 Poisson, 10,368 tetrahedra 25 us (52);
-// 2D p4 Poisson, 32 right-hand sides on 7,236 triangles 76 us (236).
+// Bound by the latency of dependent products, splits and flux arithmetic at the 8 to 16 warps per SM that
+// 255 registers leave: at 3D p4 elasticity, 24,576 tetrahedra a third of the issue slots is used, the tensor
+// pipe is busy 43 % (volume) and 24 % (facets) and DRAM 14 %.  Measured on a B200, FP32 vectors, against
+// the tile products of a whole CTA behind the tcgen05 volume kernel that stood here before: the same case
+// 172 us (volume 64, facets 115, overlapping; before 242: 82 and 160); 3D p2 elasticity, 7,986
+// tetrahedra 16.7 us (39.2); 3D p3 Poisson, 10,368 tetrahedra 18.7 us (53.0); 2D p4 Poisson, 32
+// right-hand sides on 17,712 triangles 159 us (590).
 #pragma once
 
 #include "apply_tc32.cuh"
