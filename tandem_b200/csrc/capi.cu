@@ -745,13 +745,13 @@ struct SegPlan {
 };
 
 // Chunk length: about four chunks per SM over all segments (so short vectors still occupy the
-// whole GPU), a multiple of the CTA size, between kChunkMin and kChunk entries.
+// whole GPU), a multiple of the CTA size, between `least` and kChunk entries.
 void plan_chunks(std::vector<int64_t> const& seg_begin, std::vector<int64_t> const& seg_end, std::vector<Chunk>& chunks,
-                 std::vector<int>& seg_chunk) {
+                 std::vector<int>& seg_chunk, int64_t least = kChunkMin) {
     int64_t total = 0;
     for (size_t sgi = 0; sgi < seg_begin.size(); ++sgi) total += seg_end[sgi] - seg_begin[sgi];
     const int64_t target = (total / (4 * static_cast<int64_t>(device_sm_count())) + kVecThreads - 1) / kVecThreads * kVecThreads;
-    const int64_t len = std::max<int64_t>(kChunkMin, std::min<int64_t>(kChunk, target));
+    const int64_t len = std::max<int64_t>(least, std::min<int64_t>(kChunk, target));
     chunks.clear();
     seg_chunk.assign(1, 0);
     for (size_t sgi = 0; sgi < seg_begin.size(); ++sgi) {
@@ -2404,7 +2404,7 @@ int solve_segments(tdg_op* op, const double* b, double* x, std::vector<int64_t> 
 
     std::vector<Chunk> hchunks;
     std::vector<int> hseg;
-    plan_chunks(seg_begin, seg_end, hchunks, hseg);
+    plan_chunks(seg_begin, seg_end, hchunks, hseg, gmres ? kChunkMinGm : kChunkMin);
     const int nseg = static_cast<int>(seg_begin.size());
     const size_t vec = vec_entries;
     // every carve below is rounded up to 256 bytes: one 256-byte unit of slack per carve (10 FP64
