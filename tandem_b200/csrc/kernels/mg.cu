@@ -2,6 +2,7 @@
 // block-sparse kernels read the bs x bs column-major blocks with consecutive rows on consecutive
 // threads.
 #include "mg.cuh"
+#include "dispatch.hpp"
 #include "early.cuh"
 
 #include "../../../include/tandem_b200.h"
@@ -213,54 +214,64 @@ __global__ void __launch_bounds__(kT)
 }
 
 // The P1 vectors have nrhs contiguous columns of nv * Q entries; the DG level's columns start at
-// multiples of ld0.  A row's 15 to 24 entries are dependent loads (index, then value), so eight lanes
-// share it (2,197 vertices, 3D elasticity: one thread per row 14.4 us, bound by that latency).
-constexpr int kRowLanes = 8;
-
+// multiples of ld0.  A row's 15 to 24 entries are dependent loads (index, then value), so LANES lanes
+// share it: as many as keep every row's lanes on the GPU at once (2,197 vertices, 3D elasticity: one thread
+// per row 14.4 us, bound by that latency, eight 4.3), one where the rows fill it (29,841 vertices, 32
+// columns: 39 us, eight 78).
+template <int LANES>
 __device__ __forceinline__ double row_sum(double v) {
 #pragma unroll
-    for (int o = kRowLanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
+inline int row_lanes(int64_t rows) {
+    const int64_t threads = static_cast<int64_t>(device_sm_count()) * 2048;
+    int lanes = 8;
+    while (lanes > 1 && rows * lanes > threads) lanes /= 2;
+    return lanes;
+}
+
+template <int LANES>
 __global__ void __launch_bounds__(kT)
     k_aux_apply(MgAux a, const double* __restrict__ x, const double* __restrict__ b, double* __restrict__ y,
                 int nrhs) {
     const int Q = a.Q, QQ = a.Q * a.Q;
-    const int64_t n = a.nv * Q, rows = n * nrhs, padded = (rows + 3) / 4 * 4;  // whole warps stay together
-    TDG_GRID_LOOP(gl, padded * kRowLanes) {
-        const int64_t g = gl / kRowLanes;
-        const int l = static_cast<int>(gl % kRowLanes);
+    const int64_t n = a.nv * Q, rows = n * nrhs, padded = (rows + 31) / 32 * 32;  // whole warps stay together
+    TDG_GRID_LOOP(gl, padded * LANES) {
+        const int64_t g = gl / LANES;
+        const int l = static_cast<int>(gl % LANES);
         double acc = 0.0;
         if (g < rows) {
             const int64_t col = g / n, gi = g % n;
             const int64_t v = gi / Q;
             const int p = static_cast<int>(gi % Q);
             const double* xcol = x + col * n;
-            for (int64_t k = a.ptr[v] + l; k < a.ptr[v + 1]; k += kRowLanes) {
+            for (int64_t k = a.ptr[v] + l; k < a.ptr[v + 1]; k += LANES) {
                 const double* blk = a.val + k * QQ + p * Q;
                 const double* xw = xcol + static_cast<int64_t>(a.col[k]) * Q;
                 for (int q = 0; q < Q; ++q) acc += blk[q] * xw[q];
             }
         }
-        acc = row_sum(acc);
+        acc = row_sum<LANES>(acc);
         if (g < rows && l == 0) y[g] = b ? b[g] - acc : acc;
     }
 }
 
+template <int LANES>
 __global__ void __launch_bounds__(kT)
     k_aux_restrict(MgAux a, const double* __restrict__ r0, int64_t ld0, double* __restrict__ rc, int nrhs) {
     const int Q = a.Q, bs = a.Nbf * a.Q;
-    const int64_t n = a.nv * Q, rows = n * nrhs, padded = (rows + 3) / 4 * 4;
-    TDG_GRID_LOOP(gl, padded * kRowLanes) {
-        const int64_t g = gl / kRowLanes;
-        const int l = static_cast<int>(gl % kRowLanes);
+    const int64_t n = a.nv * Q, rows = n * nrhs, padded = (rows + 31) / 32 * 32;
+    TDG_GRID_LOOP(gl, padded * LANES) {
+        const int64_t g = gl / LANES;
+        const int l = static_cast<int>(gl % LANES);
         double acc = 0.0;
         if (g < rows) {
             const int64_t col = g / n, gi = g % n;
             const int64_t v = gi / Q;
             const int p = static_cast<int>(gi % Q);
-            for (int64_t k = a.vinc_ptr[v] + l; k < a.vinc_ptr[v + 1]; k += kRowLanes) {
+            for (int64_t k = a.vinc_ptr[v] + l; k < a.vinc_ptr[v + 1]; k += LANES) {
                 const int32_t inc = a.vinc[k];
                 const int64_t e = inc / a.NV;
                 const int i = inc % a.NV;
@@ -268,7 +279,7 @@ __global__ void __launch_bounds__(kT)
                 for (int kk = 0; kk < a.Nbf; ++kk) acc += a.T[kk * a.NV + i] * r[kk];
             }
         }
-        acc = row_sum(acc);
+        acc = row_sum<LANES>(acc);
         if (g < rows && l == 0) rc[g] = acc;
     }
 }
@@ -639,15 +650,25 @@ int launch_mg_restrict(int64_t E, MgInterp ip, const double* rf, int64_t ldf, do
     return launched();
 }
 
+#define TDG_ROW_LANES(KERN, ...)                                                                  \
+    switch (row_lanes(rows)) {                                                                    \
+        case 8: KERN<8><<<grid_for(rows * 8), kT, 0, s>>>(__VA_ARGS__); break;                    \
+        case 4: KERN<4><<<grid_for(rows * 4), kT, 0, s>>>(__VA_ARGS__); break;                    \
+        case 2: KERN<2><<<grid_for(rows * 2), kT, 0, s>>>(__VA_ARGS__); break;                    \
+        default: KERN<1><<<grid_for(rows), kT, 0, s>>>(__VA_ARGS__); break;                       \
+    }
 int launch_aux_apply(MgAux const& a, const double* x, const double* b, double* y, int nrhs, cudaStream_t s) {
-    k_aux_apply<<<grid_for(a.nv * a.Q * nrhs * kRowLanes), kT, 0, s>>>(a, x, b, y, nrhs);
+    const int64_t rows = a.nv * a.Q * nrhs;
+    TDG_ROW_LANES(k_aux_apply, a, x, b, y, nrhs)
     return launched();
 }
 
 int launch_aux_restrict(MgAux const& a, const double* r0, int64_t ld0, double* rc, int nrhs, cudaStream_t s) {
-    k_aux_restrict<<<grid_for(a.nv * a.Q * nrhs * kRowLanes), kT, 0, s>>>(a, r0, ld0, rc, nrhs);
+    const int64_t rows = a.nv * a.Q * nrhs;
+    TDG_ROW_LANES(k_aux_restrict, a, r0, ld0, rc, nrhs)
     return launched();
 }
+#undef TDG_ROW_LANES
 
 int launch_aux_prolong_add(MgAux const& a, int64_t E, const double* xc, double* x0, int64_t ld0, int nrhs,
                            cudaStream_t s) {
