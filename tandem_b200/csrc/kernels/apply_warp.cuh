@@ -476,18 +476,17 @@ __global__ void __launch_bounds__(32 * WarpTile<S>::FWARPS, 1)
     const auto side_geo = [&](Item const& it, int side, int b) {
         return wg.fct + it.tile * gstride + b * (L::FF * 64) + (side ? L::SF * (b < blk.full ? 64 : 32) : 0);
     };
-    bool ok = true;  // this lane's waits have ended in time
+    unsigned late = 0;  // 2 | the phase whose wait ran out: no further waits and copies
     const auto issue = [&](Item const& it, int side, int b) {  // starts their copy into the warp's buffer
-        if (lane == 0 && ok)
+        if (lane == 0 && !late)
             bulk_load(gbuf, side_geo(it, side, b),
                       static_cast<unsigned>(facet_side_doubles<S>(b < blk.full ? 2 : 1) * sizeof(double)), &s_gbar[warp]);
     };
     unsigned parity = 0;
     const auto arrived = [&] {
-        if (ok && !mbar_wait_bounded(&s_gbar[warp], parity)) {
-            ok = false;  // no further waits and copies; the host reads the status word
+        if (!late && !mbar_wait_bounded(&s_gbar[warp], parity)) {
+            late = 2 | parity;  // the host reads the status word
             if (wg.status) atomicExch(wg.status, 1);
-            mbar_wait_bounded(&s_gbar[warp], parity);  // once more: the copy in flight must not outlive the CTA
         }
         parity ^= 1;
     };
@@ -585,6 +584,7 @@ __global__ void __launch_bounds__(32 * WarpTile<S>::FWARPS, 1)
         else
             fetch(item, it);
     }
+    if (L::STREAM && late) mbar_wait_bounded(&s_gbar[warp], late & 1);  // its copy must not outlive the CTA
 }
 
 // ---- volume term -------------------------------------------------------------------------------------
